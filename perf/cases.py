@@ -3,8 +3,9 @@
 Every case runs with per-photon random streams (photon i draws from the stream of (seed, i)),
 so that a call on the same inputs registers the same hits; the order in which hits are
 appended changes from run to run, and a reader of hits sorts them by event, DOM and time.
-Outputs are whole buffers: what lies beyond the records of a pass is zero.  Detector configurations are the synthetic ones of ppc_b200/synth.py; one context per
-configuration is kept for the whole program, as a user's program keeps its detector.
+Outputs are whole buffers: what lies beyond the records of a pass is zero.  Detector
+configurations are the synthetic ones of ppc_b200/synth.py; one context per configuration is
+kept for the whole program, as a user's program keeps its detector.
 
   kind      entry point                         what a program does there
   call      PPC.propagate                       host bunches in, host hits out
@@ -312,8 +313,8 @@ def run(s):
         info = s["batch"].run(s["bunches"], s["case"]["events"], hits_per_photon=0.05)
         produced, offsets = s["batch"].counts()
         hits = torch.from_numpy(_words(s["batch"].hits())).cuda()
-        return {"hits": _in_order(hits, s["ordered"]), "produced": produced.astype(np.int64), "offsets": offsets.astype(np.int64),
-                "steps": info["steps"]}
+        return {"hits": _in_order(hits, s["ordered"]), "produced": produced.astype(np.int64),
+                "offsets": offsets.astype(np.int64), "steps": info["steps"]}
     if kind == "gradient":
         r = c.gradient(s["bunches"], observed=s["observed"], events=s["case"]["events"])
         return {"ll": r["ll"], "counts": r["counts"].astype(np.int64), "g_be": r["g_be"], "g_ba": r["g_ba"]}
