@@ -7,8 +7,9 @@
 //     photon only when its previous one is absorbed, so the 48-byte per-photon phase-1
 //     record never round-trips through HBM;
 //   * photon indices are handed out by one warp-aggregated atomic per refill (one
-//     global counter, 64-bit, so a launch may cover more than 2^32 photons), or
-//     statically (photon i on thread i mod T) in deterministic mode;
+//     global counter, 64-bit, so a launch may cover more than 2^32 photons), photons with
+//     a large absorption depth before the others (WarpClaims), or statically (photon i on
+//     thread i mod T) in deterministic mode;
 //   * the photon -> bunch map is a binary search over an exclusive prefix sum, so a
 //     launch may hold thousands of bunches/events;
 //   * the small tables (per-layer anisotropy/BFR, strings, cell index, tilt radii) sit
@@ -1004,6 +1005,46 @@ struct PhotonPool {
   float4 n[32];
   int4 m[32];                   // wavelength bin, segment, flasher DOM, veto code
   uint4 st[STREAMS ? 32 : 1];   // per-photon streams: state x, y and multiplier index
+  float u[STREAMS ? 1 : 32];    // thread streams: the uniform number of the absorption depth, 0: not drawn yet
+};
+
+// The order in which a warp takes photons.  A photon's number of steps goes with its
+// absorption depth -log(u), so it is exponential: taken in index order, the last photons of
+// a launch leave the GPU with ever fewer live lanes for some ten mean lifetimes (350 steps
+// of 1.6-2.2 us each, 0.75 ms: half of the time of a launch of 1e6 photons).  So the first
+// photons, up to kScreenGroups per thread, are screened: a warp samples a group of 32 and at
+// once runs those with u < kScreenU (absorption depth above 2: 13.5% of them), and leaves the
+// others (a bit mask per group) to the end of the launch, when only short photons should
+// start.  Sampling a group takes the issue slots of about one step, so a screened photon,
+// sampled twice, costs 1/26 more.  Measured on the full detector's cascades without and with
+// it: 6e5 photons 1220 and 1104 us, 1e6 1634 and 1394, 3e6 3254 and 2776, 3e7 25810 and
+// 24970; 8 and 24 groups take 7% and 2% longer for 3e6, a kScreenU of 0.05 or 0.30 3% and 6%.
+// Below three photons per thread the launch lasts as long as its longest photon whenever
+// that starts (3e5 photons: 1045 us without, 1069 with it), and nothing is screened.
+constexpr int kScreenGroups = 16;
+constexpr float kScreenU = 0.135f;
+constexpr uint64_t kScreenFrom = 3;  // photons per thread
+
+// A launch of fewer photons than threads is dealt out over the SMs at its start, at best to
+// this many sixteenths of the warps (five per SM), a few lanes each: it is bound by the
+// latency of a step, 1.6 us for one lane, 2.2 us for a full warp and 3.6 us when every warp
+// of the SM is at work.  1000 photons 384 -> 283 us, 4096 630 -> 498, 3e4 785 -> 674 us
+// (with five sixteenths 4% more).
+constexpr uint32_t kFewWarps = 3;
+
+// A warp's place in that order (shared memory; read and written by lane 0's turn only).
+struct WarpClaims {
+  uint32_t left[kScreenGroups];  // screened groups: the lanes whose photon is left for the end
+  int screened, finished;        // groups screened; groups whose left-over photons were taken
+  int queue_done;                // the launch's queue (or the warp's share of few photons) has been taken
+};
+
+// The launch's sizes (per block, in shared memory: used once per photon).
+struct LaunchPlan {
+  uint64_t num;  // photons
+  int nb;        // bunches
+  int groups;    // screened groups per warp
+  int deal;      // fewer photons than threads: photons per warp, dealt at the start; else -1
 };
 
 // Random streams.  Thread streams (STREAMS = false, the reference's scheme): each thread
@@ -1026,18 +1067,30 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   PhotonPool<STREAMS>* pools = reinterpret_cast<PhotonPool<STREAMS>*>(dsm);
   Prov* snaps = reinterpret_cast<Prov*>(dsm + (BLOCK / 32) * sizeof(PhotonPool<STREAMS>));
   __shared__ unsigned long long bsteps;  // the block's propagation steps
-  if (threadIdx.x == 0) bsteps = 0;
+  __shared__ WarpClaims s_claims[BLOCK / 32];
+  __shared__ LaunchPlan plan;
+  if (threadIdx.x == 0) {
+    bsteps = 0;
+    const uint32_t T = gridDim.x * BLOCK, few = max(1u, T / 32 * kFewWarps / 16);
+    // launch sizes: from the parameters, or from device memory for replayed graphs
+    plan.num = a.dyn ? a.dyn[0] : a.num;
+    plan.nb = a.dyn ? (int)a.dyn[1] : a.nb;
+    plan.groups = plan.num >= kScreenFrom * T ? (int)min((uint64_t)kScreenGroups, plan.num / T) : 0;
+    plan.deal = plan.num < T ? (int)min((uint64_t)32, (plan.num + few - 1) / few) : -1;
+  }
+  if (threadIdx.x < BLOCK / 32) {
+    WarpClaims& c = s_claims[threadIdx.x];
+    c.screened = c.finished = c.queue_done = 0;
+  }
   load_tables(a, S);
   const DynTabs dt = load_dyn(a, dsm + dyn_smem<BLOCK, REC, STREAMS>());
-  // launch sizes: from the parameters, or from device memory for replayed graphs
-  const uint64_t num = a.dyn ? a.dyn[0] : a.num;
-  const int nb = a.dyn ? (int)a.dyn[1] : a.nb;
   const uint32_t T = gridDim.x * blockDim.x;
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t nmul = T < 1024u ? T : 1024u;  // multipliers used by per-photon streams
   const unsigned int lane = threadIdx.x & 31;
   const unsigned int FULL = 0xffffffffu;
   PhotonPool<STREAMS>& P = pools[threadIdx.x >> 5];
+  WarpClaims& C = s_claims[threadIdx.x >> 5];
   Rng s;
   uint32_t mi = gt;  // multiplier index of the stream in s
   {
@@ -1046,7 +1099,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   }
   Photon ph;
   bool alive = false;
-  bool exhausted = false;   // warp-uniform: no photons left to sample
+  bool done = false;        // warp-uniform: no photons left to sample
   int have = 0;             // warp-uniform: photons in the pool
   // rarely used per-thread state in shared memory instead of registers: the next photon
   // index in the static order and the last bunch found
@@ -1066,97 +1119,136 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   // every lane of the warp stays in this loop until the warp is done, so the warp-wide
   // operations below always see all 32 lanes
   while (true) {
-    const unsigned int dead = __ballot_sync(FULL, !alive);
-    if (dead && !(exhausted && have == 0)) {
+    unsigned int dead = __ballot_sync(FULL, !alive);
+    float u_abs = 0;  // thread streams: the absorption depth's uniform number, when drawn at sampling
+    while (dead && !done) {
       // --- sample: each generating lane produces one photon
-      bool gen = false;
-      uint64_t gidx = 0;
-      unsigned long long base = 0;
-      int ngen = 0;
-      if (a.deterministic == 1) {  // photon i on thread i mod T, as the oracle sequences it
-        gen = !alive && s_sidx[threadIdx.x] < num;
-        gidx = s_sidx[threadIdx.x];
-        if (!alive) s_sidx[threadIdx.x] += T;
-      } else if ((have < __popc(dead) || have < a.refill_below) && !exhausted) {
-        ngen = 32 - have;
-        if (lane == 0) base = atomicAdd(&a.ctrl->next, (unsigned long long)ngen);
-        base = __shfl_sync(FULL, base, 0);
-        gidx = base + lane;
-        gen = (int)lane < ngen && gidx < num;
-        if (base + ngen >= num) exhausted = true;
-      }
-      Photon g;
-      uint4 gst = make_uint4(0, 0, 0, 0);
-      if (gen) {
-        const int hint = find_bunch(a, nb, gidx, s_hint[threadIdx.x]);
-        s_hint[threadIdx.x] = hint;
-        if constexpr (STREAMS) {  // the photon's own stream; the lane's s is left alone
-          Rng sg;
-          const uint32_t m = (uint32_t)(gidx % nmul);
-          sg.a = a.rm[m];
-          photon_stream(sg, gidx, a.seed);
-          const Sampled smp = sample_photon(a, hint, sg.x, sg.y, sg.a);
-          g = smp.ph;
-          gst = make_uint4(smp.x, smp.y, m, 0);
-        } else {
-          const Sampled smp = sample_photon(a, hint, s.x, s.y, s.a);
-          g = smp.ph;
-          s.x = smp.x; s.y = smp.y;
+      const bool fixed = a.deterministic == 1;
+      if (fixed || have == 0 || have < a.refill_below) {
+        bool gen = false, screen = false, late = false, last = false;
+        uint64_t gidx = 0;
+        float u = 0;
+        // warps are numbered across the blocks first, so that few photons spread over all SMs
+        const uint32_t warps = T >> 5, gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        if (fixed) {  // photon i on thread i mod T, as the oracle sequences it
+          gen = !alive && s_sidx[threadIdx.x] < plan.num;
+          gidx = s_sidx[threadIdx.x];
+          if (!alive) s_sidx[threadIdx.x] += T;
+          done = __all_sync(FULL, s_sidx[threadIdx.x] >= plan.num);
+        } else if (C.screened < plan.groups) {  // the next group to screen, once the pool is empty
+          gen = screen = have == 0;
+          gidx = ((uint64_t)C.screened * warps + gw) * 32 + lane;
+        } else if (!C.queue_done) {  // the warp's share of few photons, or the queue
+          const int n = plan.deal >= 0 ? plan.deal : 32 - have;
+          unsigned long long base = (uint64_t)gw * n;
+          if (plan.deal < 0) {
+            if (lane == 0) base = atomicAdd(&a.ctrl->next, (unsigned long long)n);
+            base = (uint64_t)plan.groups * T + __shfl_sync(FULL, base, 0);
+          }
+          last = plan.deal >= 0 || base + n >= plan.num;
+          gidx = base + lane;
+          gen = (int)lane < n && gidx < plan.num;
+        } else if (have == 0 && C.finished < plan.groups) {  // photons left over by the screening
+          late = true;
+          gen = C.left[C.finished] >> lane & 1u;
+          gidx = ((uint64_t)C.finished * warps + gw) * 32 + lane;
+          if constexpr (!STREAMS) u = fmaf(1 - kScreenU, xrnd(s), kScreenU);
+        } else if (have == 0) {
+          done = true;
+          break;
         }
-      }
-      if (a.deterministic == 1) {
-        if (gen) {
-          ph = g;
-          alive = true;
-          if constexpr (STREAMS) { s.x = gst.x; s.y = gst.y; mi = gst.z; s.a = a.rm[mi]; }
+        if constexpr (!STREAMS) {
+          if (screen) {  // the decision comes first: only the photons that run now are sampled
+            u = xrnd(s);
+            gen = u < kScreenU;
+          }
         }
-        exhausted = __all_sync(FULL, s_sidx[threadIdx.x] >= num);
-      } else {
+        __syncwarp();  // C has been read by all lanes
+        Photon g;
+        uint4 gst = make_uint4(0, 0, 0, 0);
         if (gen) {
-          const int slot = have + lane;
+          const int hint = find_bunch(a, plan.nb, gidx, s_hint[threadIdx.x]);
+          s_hint[threadIdx.x] = hint;
+          if constexpr (STREAMS) {  // the photon's own stream; the lane's s is left alone
+            Rng sg;
+            const uint32_t m = (uint32_t)(gidx % nmul);
+            sg.a = a.rm[m];
+            photon_stream(sg, gidx, a.seed);
+            const Sampled smp = sample_photon(a, hint, sg.x, sg.y, sg.a);
+            g = smp.ph;
+            gst = make_uint4(smp.x, smp.y, m, 0);
+            if (screen) {  // the number that the pick-up below turns into the absorption depth
+              sg.x = smp.x; sg.y = smp.y;
+              gen = xrnd(sg) < kScreenU;
+            }
+          } else {
+            const Sampled smp = sample_photon(a, hint, s.x, s.y, s.a);
+            g = smp.ph;
+            s.x = smp.x; s.y = smp.y;
+          }
+        }
+        if (fixed) {
+          if (gen) {
+            ph = g;
+            ph.TOT = -1;
+            alive = true;
+            if constexpr (STREAMS) { s.x = gst.x; s.y = gst.y; mi = gst.z; s.a = a.rm[mi]; }
+          }
+          break;
+        }
+        const unsigned int kept = __ballot_sync(FULL, gen);
+        if (gen) {
+          const int slot = have + __popc(kept & ((1u << lane) - 1u));
           P.r[slot] = g.r;
           P.n[slot] = g.n;
           P.m[slot] = make_int4(g.wl, (int)g.niw, g.om0, g.ofla);
           if constexpr (STREAMS) P.st[slot] = gst;
+          else P.u[slot] = u;
         }
-        have += __popc(__ballot_sync(FULL, gen));
-        __syncwarp();
-        // --- hand out: the k-th dead lane takes the k-th photon from the top of the pool
-        const int rank = __popc(dead & ((1u << lane) - 1u));
-        if (!alive && rank < have) {
-          const int slot = have - 1 - rank;
-          ph.r = P.r[slot];
-          ph.n = P.n[slot];
-          const int4 m = P.m[slot];
-          ph.wl = m.x; ph.niw = (uint32_t)m.y; ph.om0 = m.z; ph.ofla = m.w;
-          if constexpr (STREAMS) {
-            const uint4 t = P.st[slot];
-            s.x = t.x; s.y = t.y; mi = t.z; s.a = a.rm[mi];
-          }
-          alive = true;
+        if (lane == 0) {
+          if (screen) C.left[C.screened++] = ~kept;
+          if (last) C.queue_done = 1;
+          if (late) C.finished++;
         }
-        have -= min(have, __popc(dead));
+        have += __popc(kept);
         __syncwarp();
       }
-      if (alive && (dead >> lane & 1u)) {  // a fresh photon: absorption depth, gpu/pro.cu:496-497
-        ph.nhit = 0;
-        if constexpr (REC) {
-          hk.start->r = ph.r;
-          hk.start->n = ph.n;
-          hk.start->m = make_int4(ph.wl, (int)ph.niw, ph.om0, ph.ofla);
-          hk.start->s = make_uint4(s.x, s.y, mi, 0);
+      // --- hand out: the k-th dead lane takes the k-th photon from the top of the pool
+      const int rank = __popc(dead & ((1u << lane) - 1u));
+      if (!alive && rank < have) {
+        const int slot = have - 1 - rank;
+        ph.r = P.r[slot];
+        ph.n = P.n[slot];
+        const int4 m = P.m[slot];
+        ph.wl = m.x; ph.niw = (uint32_t)m.y; ph.om0 = m.z; ph.ofla = m.w;
+        if constexpr (STREAMS) {
+          const uint4 t = P.st[slot];
+          s.x = t.x; s.y = t.y; mi = t.z; s.a = a.rm[mi];
+        } else {
+          u_abs = P.u[slot];
         }
-        ph.TOT = -logf(xrnd(s));
-        ph.SCA = 0;
-        ph.old = -1;
-        ph.steps = 0;
-        if (ph.ofla < -1) ph.TOT = 0;
+        ph.TOT = -1;
+        alive = true;
       }
+      have -= min(have, __popc(dead));
+      dead = __ballot_sync(FULL, !alive);
     }
-    if (!__any_sync(FULL, alive)) {
-      if (exhausted && have == 0) break;
-      continue;
+    if (alive && ph.TOT < 0) {  // a fresh photon: absorption depth, gpu/pro.cu:496-497
+      ph.nhit = 0;
+      if constexpr (REC) {
+        hk.start->r = ph.r;
+        hk.start->n = ph.n;
+        hk.start->m = make_int4(ph.wl, (int)ph.niw, ph.om0, ph.ofla);
+        hk.start->s = make_uint4(s.x, s.y, mi, 0);
+      }
+      if (u_abs == 0) u_abs = xrnd(s);
+      ph.TOT = -logf(u_abs);
+      ph.SCA = 0;
+      ph.old = -1;
+      ph.steps = 0;
+      if (ph.ofla < -1) ph.TOT = 0;
     }
+    if (!__any_sync(FULL, alive)) break;
     if (alive) {
       step(a, S, dt, ph, s, nan_steps, hk);
       ph.steps++;
