@@ -11,15 +11,29 @@ namespace ppcb {
 
 constexpr int kMaxPoly = 16;
 
-struct BackDom {
+// What a hit's decision needs of its sensor: one 32-byte load (the lanes' hits lie on
+// different DOMs, so every load instruction gathers).  The key (str, om) has its own table.
+struct __align__(32) BackDom {
+  float scale;      // rde / rmax
+  int16_t acc;      // acceptance table, -1: never registers (no HV, no table, rde = 0)
+  int16_t sensor;   // sensor type, -1: none
+  float R, F;       // radius and spheroid factor
   float tilt[3];
   float azi;        // cable azimuth [deg], < 0: none
-  float R, F;       // radius and spheroid factor
-  float scale;      // rde / rmax
-  int acc;          // acceptance table, -1: never registers (no HV, no table, rde = 0)
-  int sensor;       // sensor type, -1: none
-  int str, om;
 };
+static_assert(sizeof(BackDom) == 32, "one 32-byte load");
+
+// 32 bytes from a 32-byte boundary through the read-only path, in one instruction (sm_100).
+struct Words8 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ Words8 load32(const void* p) {
+  Words8 v;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
+      : "l"(p));
+  return v;
+}
 
 // Sensor kinds of getPMT (gpu/ini.cxx:210-280)
 constexpr int kSensorStandard = 0;  // one PMT: angular polynomial or impact-height threshold
@@ -49,13 +63,29 @@ struct BackArgs {
   const ppcb_hit* hits;
   uint64_t n;
   const BackDom* doms;
+  const int2* keys;     // str, om
   const BackSensor* sensors;
   const float* rat;     // [acceptance tables][WNUM]
   const float3* dirs;   // PMT axes of the multi-PMT sensors
   const float2* wvs;    // [WNUM] bin edges (i, f)
   const uint32_t* rm;
   uint32_t nmul, seed, gsize;
+  int wide;             // hits lie on a 32-byte boundary
 };
+
+// A caller's hit record: one 32-byte load where its address allows it.
+__device__ __forceinline__ ppcb_hit load_hit(const BackArgs& A, uint64_t k) {
+  ppcb_hit h;
+  if (A.wide) {
+    const Words8 v = load32(A.hits + k);
+    h.i = v.w[0]; h.n = v.w[1]; h.z = v.w[2]; h.t = __uint_as_float(v.w[3]);
+    h.pth = __uint_as_float(v.w[4]); h.pph = __uint_as_float(v.w[5]);
+    h.dth = __uint_as_float(v.w[6]); h.dph = __uint_as_float(v.w[7]);
+  } else {
+    h = A.hits[k];
+  }
+  return h;
+}
 
 // angular response of one PMT to light arriving at cos(angle) x off its axis (itype::f,
 // gpu/ini.cxx:173-187): the projected area of a disc behind a sphere segment of opening beta
@@ -130,20 +160,30 @@ __device__ __forceinline__ int tube_pmt(const BackSensor& S, float rz, float u, 
   return i;
 }
 
-// decides hit k; fills `o` when accepted
-__device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_acc_hit& o) {
-  const ppcb_hit h = A.hits[k];
+// Decides hit k; fills `o` when accepted.  DECIDED: the hit has been accepted before, on PMT
+// `known` (-1: not kept); the record is filled without the tests, which another instance of
+// this code may have rounded differently.
+template <bool DECIDED = false>
+__device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_acc_hit& o, int known = -1) {
+  const ppcb_hit h = load_hit(A, k);
   if (h.i >= A.gsize || h.z >= PPCB_WNUM) return false;
-  const BackDom D = A.doms[h.i];
-  if (D.acc < 0) return false;
+  const Words8 d = load32(A.doms + h.i);
+  BackDom D;
+  D.scale = __uint_as_float(d.w[0]); D.acc = (int16_t)d.w[1]; D.sensor = (int16_t)(d.w[1] >> 16);
+  D.R = __uint_as_float(d.w[2]); D.F = __uint_as_float(d.w[3]);
+  for (int j = 0; j < 3; j++) D.tilt[j] = __uint_as_float(d.w[4 + j]);
+  D.azi = __uint_as_float(d.w[7]);
+  if (D.acc < 0 || D.sensor < 0) return false;
   // the hit's stream: a SplitMix64 hash (Steele, Lea, Flood 2014) of (seed, k)
   uint64_t z = ((uint64_t)A.seed << 32 | 0x6a09e667u) + (k + 1) * 0x9e3779b97f4a7c15ull;
   z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
   z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
   z ^= z >> 31;
-  const uint32_t a = A.rm[k % A.nmul];
+  const uint32_t im = (A.nmul & (A.nmul - 1)) ? (uint32_t)(k % A.nmul) : (uint32_t)k & (A.nmul - 1);
+  const uint32_t a = __ldg(&A.rm[im]);
   uint32_t sx = (uint32_t)z, sy = __umulhi((uint32_t)(z >> 32), a);
-  if (!(bxrnd(sx, sy, a) < A.rat[(size_t)D.acc * PPCB_WNUM + h.z] * D.scale)) return false;
+  const float u0 = bxrnd(sx, sy, a);
+  if (!DECIDED && !(u0 < __ldg(&A.rat[(size_t)D.acc * PPCB_WNUM + h.z]) * D.scale)) return false;
   float ptc, pts, ppc, pps, dpc, dps;
   sincosf(h.pth, &pts, &ptc);
   sincosf(h.pph, &pps, &ppc);
@@ -152,12 +192,16 @@ __device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_a
   const float dts = D.F < 0 ? 1.f : sinf(h.dth);
   const float rx = dts * dpc, ry = dts * dps, rz = dtc;
   const float nx = pts * ppc, ny = pts * pps, nz = ptc;
-  if (D.sensor < 0) return false;
   const BackSensor& S = A.sensors[D.sensor];
   const float u = bxrnd(sx, sy, a);
   int pmt = 0;
   float t = h.t;
-  if (S.kind == kSensorStandard) {
+  if (S.kind == kSensorMultiPMT) {
+    pmt = DECIDED ? known : multi_pmt(A, S, D.azi, nx, ny, nz, u);
+    if (!DECIDED && pmt < 0) return false;
+  } else if (S.kind == kSensorTube) {
+    pmt = tube_pmt(S, rz, u, t, sx, sy, a);
+  } else if (!DECIDED) {
     bool flag;
     if (S.mas > 0) {
       const float x = nx * D.tilt[0] + ny * D.tilt[1] + nz * D.tilt[2];
@@ -168,13 +212,8 @@ __device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_a
       flag = rx * D.tilt[0] + ry * D.tilt[1] + rz * D.tilt[2] > S.s[0];
     }
     if (!flag) return false;
-  } else if (S.kind == kSensorMultiPMT) {
-    pmt = multi_pmt(A, S, D.azi, nx, ny, nz, u);
-    if (pmt < 0) return false;
-  } else {
-    pmt = tube_pmt(S, rz, u, t, sx, sy, a);
   }
-  if (D.azi >= 0) {  // cable shadow
+  if (!DECIDED && D.azi >= 0) {  // cable shadow
     const float rc = 0.023f, dc = D.R + rc;
     float sp, cp;
     sincosf(D.azi * (PPCB_FPI / 180.f), &sp, &cp);
@@ -187,9 +226,10 @@ __device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_a
       if (Dd >= 0 && (-b + sqrtf(Dd)) / (2 * aa) > 0) return false;
     }
   }
-  const float2 w = A.wvs[h.z];
+  const int2 key = __ldg(&A.keys[h.i]);
+  const float2 w = __ldg(&A.wvs[h.z]);
   o.i = h.i; o.n = h.n; o.hit = (uint32_t)k;
-  o.str = D.str; o.om = D.om; o.pmt = pmt;
+  o.str = key.x; o.om = key.y; o.pmt = pmt;
   o.t = t;
   o.wv = w.x + (w.y - w.x) * bxrnd(sx, sy, a);
   o.r[0] = -D.R * rx; o.r[1] = -D.R * ry; o.r[2] = -D.R * rz;
@@ -199,16 +239,22 @@ __device__ __forceinline__ bool accept_one(const BackArgs& A, uint64_t k, ppcb_a
 
 struct BackendTables {
   BackDom* doms = nullptr;
+  int2* keys = nullptr;
   BackSensor* sensors = nullptr;
   float* rat = nullptr;
   float2* wvs = nullptr;
   float3* dirs = nullptr;
-  unsigned int* block_cnt = nullptr;
-  unsigned long long* block_off = nullptr;
-  uint64_t blocks_cap = 0;
+  // a call's scratch (backend.cu): per tile of hits the accepted ones' number and offset, per
+  // hit a bit
+  unsigned long long* tile_off = nullptr;
+  unsigned int* tile_cnt = nullptr;
+  uint32_t* bits = nullptr;
+  uint16_t* pmts = nullptr;  // PMTs of the accepted hits, where there are multi-PMT sensors
+  bool multi_pmt = false;
+  uint64_t tiles_cap = 0;
   ~BackendTables() {
-    for (void* p : {(void*)doms, (void*)sensors, (void*)rat, (void*)wvs, (void*)dirs, (void*)block_cnt,
-                    (void*)block_off})
+    for (void* p : {(void*)doms, (void*)keys, (void*)sensors, (void*)rat, (void*)wvs, (void*)dirs, (void*)tile_off,
+                    (void*)tile_cnt, (void*)bits, (void*)pmts})
       if (p) cudaFree(p);
   }
 };
