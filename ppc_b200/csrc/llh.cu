@@ -1,20 +1,23 @@
-// Simulated side of DirectFit's likelihood on the GPU, three kernels per evaluation:
-//   k_llh_fill    one thread per kernel-level hit: the back end's acceptance (backend.cuh,
-//                 the same per-hit streams as Engine::accept), then for each time shift the
-//                 hit's bin round((t + dt - t0) / lbin) and, when it lies in the DOM's
-//                 window and outside its errata windows, +1 on that bin's block (dat::fill,
-//                 dat::join, llh/llh.cxx:469-482, 614-621).  Simulated hits on DOMs without
-//                 observed pulses count toward the no-hit total (cascade::ppc,
-//                 llh/llh.cxx:1694-1700).
+// Simulated side of DirectFit's likelihood on the GPU:
+//   k_llh_count   per kernel-level hit the back end's acceptance (backend.cuh, the same
+//                 per-hit streams as Engine::accept), then for each time shift the hit's bin
+//                 round((t + dt - t0) / lbin) and, when it lies in the DOM's window and
+//                 outside its errata windows, +1 on that bin's block (dat::fill, dat::join,
+//                 llh/llh.cxx:469-482, 614-621), in the block's own counters in shared
+//                 memory.  Simulated hits on DOMs without observed pulses count toward the
+//                 no-hit total (cascade::ppc, llh/llh.cxx:1694-1700).
+//   k_llh_accept  when the counters of all shifts do not fit: the acceptance alone, once,
+//                 for k_llh_count to run over parts of the shifts.
 //   k_llh_terms   one thread per (shift, block): llf (llh/llh.cxx:637-662) in FP64, a
-//                 fixed-order tree sum per CTA.
-//   k_llh_final   one CTA per shift: the CTA sums in a fixed order, the no-hit term and the
-//                 division by ndof (fllh, llh/llh.cxx:1075-1082).
+//                 fixed-order tree sum per CTA; the last CTA of a shift adds the CTA sums in
+//                 a fixed order, the no-hit term and divides by ndof (fllh,
+//                 llh/llh.cxx:1075-1082).
 // Counts are integers (one per accepted hit), so the binning is exact; every sum runs in a
 // fixed order, so an evaluation is deterministic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "backend.cuh"
@@ -30,15 +33,17 @@ struct LlhDevice {
   double* block_dat = nullptr;
   int32_t* block_dom = nullptr;
   double2* win = nullptr;
-  unsigned int* simc = nullptr;      // [shift][block] simulated counts
-  unsigned int* stot = nullptr;      // [shift][DOM] simulated counts in the DOM's window
-  unsigned long long* nohit = nullptr;
+  // counters of an evaluation, cleared by one memset: the no-hit total, one ticket per shift,
+  // simulated counts [block][shift], and (norm) counts in the DOMs' windows [DOM][shift]
+  unsigned int* work = nullptr;
   double* partial = nullptr;         // [shift][CTA] sums of llf terms
   int* errors = nullptr;
   int ndt_cap = 0;
+  float2* list = nullptr;            // accepted hits (slot, time) of an evaluation in parts
+  uint64_t list_cap = 0;
   ~LlhDevice() {
     for (void* p : {(void*)dom_slot, (void*)doms, (void*)bin_block, (void*)block_dat, (void*)block_dom, (void*)win,
-                    (void*)simc, (void*)stot, (void*)nohit, (void*)partial, (void*)errors})
+                    (void*)work, (void*)partial, (void*)errors, (void*)list})
       if (p) cudaFree(p);
   }
 };
@@ -50,49 +55,152 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kMaxNewton = 200;
 
-struct FillArgs {
+constexpr int kCountThreads = 1024;
+constexpr size_t kCountSmem = 192 << 10;  // shared memory of the counters of one CTA, at most
+
+struct CountArgs {
   BackArgs A;
   const int32_t* dom_slot;
   const LlhDom* doms;
   const int32_t* bin_block;
   const double2* win;
-  unsigned int* simc;
-  unsigned int* stot;
+  const float2* list;   // accepted hits instead of A's (evaluation in parts)
+  unsigned int* simc;   // [block][shift]
+  unsigned int* stot;   // [DOM][shift]
   unsigned long long* nohit;
   double t0, lbin;
-  int nblocks, ndom, ndt, unh, norm;
+  int nblocks, ndt, unh, norm;
+  int j0, nj;           // the part's shifts [j0, j0 + nj) of ndt
+  int smem;             // the counters are in shared memory
   double dt[PPCB_LLH_MAX_SHIFTS];
 };
 
-__global__ void __launch_bounds__(kThreads) k_llh_fill(FillArgs F) {
-  __shared__ unsigned int s_nohit;
-  if (threadIdx.x == 0) s_nohit = 0;
-  __syncthreads();
-  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+// What a lane knows of its accepted hit.
+struct BinnedHit {
+  int slot;       // DOM slot; -1: no observed pulses there, -2: not accepted or left out
+  float t;
+};
+
+__device__ __forceinline__ BinnedHit llh_hit(const BackArgs& A, const int32_t* dom_slot, uint64_t k) {
+  BinnedHit h{-2, 0.f};
   ppcb_acc_hit o;
-  if (k < F.A.n && accept_one(F.A, k, o)) {
-    const int slot = F.dom_slot[o.i];
-    if (slot == -1) {
-      if (F.unh) atomicAdd(&s_nohit, 1u);
-    } else if (slot >= 0) {
-      const LlhDom D = F.doms[slot];
-      for (int j = 0; j < F.ndt; j++) {
-        const double t = (double)o.t + F.dt[j];
-        bool ok = true;
-        for (int w = 0; w < D.nwin; w++) {
-          const double2 x = F.win[D.win0 + w];
-          if (x.x <= t && t < x.y) ok = false;
-        }
-        if (!ok) continue;
-        const double b = round((t - F.t0) / F.lbin);
-        if (!(b >= D.n1 && b < D.n2)) continue;  // also drops NaN times
-        const int blk = F.bin_block[D.bin0 + (int)b - D.n1];
-        atomicAdd(&F.simc[(size_t)j * F.nblocks + blk], 1u);
-        if (F.norm) atomicAdd(&F.stot[(size_t)j * F.ndom + slot], 1u);  // only norm reads it
-      }
-    }
+  if (k < A.n && accept_one(A, k, o)) {
+    h.slot = dom_slot[o.i];
+    h.t = o.t;
+  }
+  return h;
+}
+
+__global__ void __launch_bounds__(kThreads) k_llh_accept(BackArgs A, const int32_t* dom_slot, float2* list) {
+  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+  const BinnedHit h = llh_hit(A, dom_slot, k);
+  if (k < A.n) list[k] = make_float2(__int_as_float(h.slot), h.t);
+}
+
+// The reference's bin of time t shifted by dt, relative to the DOM's window: in [0, n2 - n1)
+// when the hit takes part.  `q` is the quotient in single precision, a sum of two numbers
+// below kMaxQuot (or a NaN), so within 1.5e-3 of it: at least 2e-3 from the middle between
+// two bins it decides; otherwise, and always with errata windows, the double-precision
+// expressions of llh/llh.cxx:469-482 do.
+constexpr float kMaxQuot = 4000.f;
+__device__ __forceinline__ float quot_part(float q) { return fabsf(q) < kMaxQuot ? q : __int_as_float(0x7fffffff); }
+
+__device__ __forceinline__ int llh_bin(const CountArgs& F, float q, float t, double dt, int n1, int n2, int win0,
+                                       int nwin) {
+  const float near = q + 12582912.f;  // 1.5 x 2^23: the nearest integer in the low mantissa bits
+  if (fabsf(q - (near - 12582912.f)) < 0.498f && nwin == 0)
+    return __float_as_int(near) - 0x4b400000 - n1;
+  const double x = (double)t + dt;
+  for (int w = 0; w < nwin; w++) {
+    const double2 e = F.win[win0 + w];
+    if (e.x <= x && x < e.y) return -1;
+  }
+  const double b = round((x - F.t0) / F.lbin);
+  return b >= n1 && b < n2 ? (int)b - n1 : -1;  // also drops NaN times
+}
+
+// An accepted hit on a DOM with observed pulses, as the warp shares it out.
+struct __align__(16) SharedHit {
+  float t, q;             // time; its part of the quotient
+  int slot, base;         // DOM slot; the DOM's bins in the bin -> block table
+  int n1, n2, win0, nwin; // bins that take part, errata windows
+};
+
+// A thread accepts a hit; then the warp takes its accepted hits a few at a time, 2^k lanes
+// per hit and a lane per shift, so that the lanes have work whatever was accepted and the
+// counters of a hit's shifts lie side by side ([block][shift]: no bank conflicts, where
+// hits of one block in all lanes would queue for one counter).  What bounds it is
+// instruction issue: the acceptance (about 250 instructions per hit) and about 15 per
+// (accepted hit, shift), against 60 of one thread's loop with a double-precision division and
+// a global atomic each.  Whole evaluation, 1.38e6 hits (0.55e6 accepted): 64 shifts 222 ->
+// 58 us, 16 shifts 90 -> 43, 5 shifts 63 -> 41, one 50 -> 39.
+template <bool LIST>
+__global__ void __launch_bounds__(kCountThreads, 1) k_llh_count(const __grid_constant__ CountArgs F) {
+  extern __shared__ unsigned int cnt[];
+  __shared__ unsigned int s_nohit;
+  __shared__ double s_dt[PPCB_LLH_MAX_SHIFTS];
+  __shared__ float s_q[PPCB_LLH_MAX_SHIFTS];
+  const float inv = (float)(1 / F.lbin);
+  __shared__ SharedHit s_hits[kCountThreads];
+  SharedHit* mine = s_hits + (threadIdx.x & ~31);
+  const int group = F.nj > 16 ? 32 : F.nj > 8 ? 16 : F.nj > 4 ? 8 : F.nj > 1 ? 4 : 1;  // lanes per hit
+  const int counters = F.nblocks * F.nj;
+  if (F.smem)
+    for (int i = threadIdx.x; i < counters; i += kCountThreads) cnt[i] = 0;
+  if (threadIdx.x == 0) s_nohit = 0;
+  if (threadIdx.x < F.nj) {
+    s_dt[threadIdx.x] = F.dt[F.j0 + threadIdx.x];
+    s_q[threadIdx.x] = quot_part((float)s_dt[threadIdx.x] * inv);
   }
   __syncthreads();
+  const unsigned int lane = threadIdx.x & 31;
+  unsigned int nohit = 0;
+  auto add = [&](int bin, int base, int slot, int j) {
+    const int blk = F.bin_block[base + bin];
+    if (F.smem) atomicAdd(&cnt[blk * F.nj + j], 1u);
+    else atomicAdd(&F.simc[(size_t)blk * F.ndt + F.j0 + j], 1u);
+    if (F.norm) atomicAdd(&F.stot[(size_t)slot * F.ndt + F.j0 + j], 1u);  // only norm reads it
+  };
+  const uint64_t tiles = (F.A.n + 31) / 32, warps = (uint64_t)gridDim.x * (kCountThreads / 32);
+  for (uint64_t tile = (uint64_t)blockIdx.x * (kCountThreads / 32) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
+    const uint64_t k = tile * 32 + lane;
+    BinnedHit h{-2, 0.f};
+    if constexpr (LIST) {
+      if (k < F.A.n) {
+        const float2 v = F.list[k];
+        h = BinnedHit{__float_as_int(v.x), v.y};
+      }
+    } else {
+      h = llh_hit(F.A, F.dom_slot, k);
+    }
+    if (F.unh && F.j0 == 0 && h.slot == -1) nohit++;
+    const unsigned int m = __ballot_sync(0xffffffffu, h.slot >= 0);
+    if (h.slot >= 0) {
+      const LlhDom& D = F.doms[h.slot];
+      mine[__popc(m & ((1u << lane) - 1u))] =
+          SharedHit{h.t, quot_part((float)((double)h.t - F.t0) * inv), h.slot, D.bin0, D.n1, D.n2, D.win0, D.nwin};
+    }
+    __syncwarp();
+    const int hits = __popc(m);
+    for (int i = lane / group; i < hits; i += 32 / group) {
+      const SharedHit x = mine[i];
+      for (int j = lane & (group - 1); j < F.nj; j += group) {
+        const int bin = llh_bin(F, x.q + s_q[j], x.t, s_dt[j], x.n1, x.n2, x.win0, x.nwin);
+        if ((unsigned)bin < (unsigned)(x.n2 - x.n1)) add(bin, x.base, x.slot, j);
+      }
+    }
+    __syncwarp();
+  }
+  if (nohit) atomicAdd(&s_nohit, nohit);
+  __syncthreads();
+  if (F.smem)
+    for (int i = threadIdx.x; i < counters; i += kCountThreads) {
+      const unsigned int c = cnt[i];
+      if (c) {
+        const int blk = i / F.nj;
+        atomicAdd(&F.simc[(size_t)blk * F.ndt + F.j0 + (i - blk * F.nj)], c);
+      }
+    }
   if (threadIdx.x == 0 && s_nohit) atomicAdd(F.nohit, (unsigned long long)s_nohit);
 }
 
@@ -107,16 +215,18 @@ __device__ double llf(double s, double d, double nsim, double ndat, double sig, 
     return nan;
   }
   if (s == 0 && d == 0) return 0;
-  const double s2 = sig * sig, tol = 1.e-8;
+  const double s2 = sig * sig, is2 = 1 / s2, tol = 1.e-8;
   const double sd = s + d, ntot = ndat + nsim;
   double ls = sd / ntot, ld = ls, llx = 0;
   if (sig > 0) {
     double dls;
     int it = 0;
     do {
-      const double f = nsim * ls - s - log(ld / ls) / s2;
-      const double df = 1 + (1 / (ndat * ld) + 1 / (nsim * ls)) / s2;
-      dls = -f / (nsim * df);
+      // the reference's step -f / (nsim (1 + (1 / b + 1 / a) / s2)) with a + b = s + d, over one
+      // denominator: two divisions per iteration instead of six
+      const double a = nsim * ls, b = ndat * ld;
+      const double f = a - s - log(ld / ls) * is2;
+      dls = -f * (a * b) / (nsim * (a * b + sd * is2));
       ls += dls;
       ld = (sd - nsim * ls) / ndat;
       if (ls < 0 || ld < 0 || ++it > kMaxNewton) {
@@ -144,53 +254,59 @@ __device__ double cta_sum(double v, double* sh) {
 }
 
 struct TermArgs {
-  const unsigned int* simc;
-  const unsigned int* stot;
+  const unsigned int* simc;   // [block][shift]
+  const unsigned int* stot;   // [DOM][shift]
+  const unsigned long long* nohit;
+  unsigned int* ticket;       // [shift] CTAs done
   const double* block_dat;
   const int32_t* block_dom;
   const LlhDom* doms;
   double* partial;
   int* errors;
+  double* out;
   double nsim, ndat, sig;
-  int nblocks, ndom, norm;
+  int nblocks, ndom, ndt, norm, ndof;
 };
 
 __global__ void __launch_bounds__(kThreads) k_llh_terms(TermArgs T) {
   __shared__ double sh[kThreads];
+  __shared__ bool last;
   const int b = blockIdx.x * kThreads + threadIdx.x, j = blockIdx.y;
   double v = 0;
   bool err = false;
   if (b < T.nblocks) {
-    const double s = T.simc[(size_t)j * T.nblocks + b];
+    const double s = T.simc[(size_t)b * T.ndt + j];
     double nsim = T.nsim;
     bool use = true;
     if (T.norm) {
       const int slot = T.block_dom[b];
-      const double st = T.stot[(size_t)j * T.ndom + slot];
+      const double st = T.stot[(size_t)slot * T.ndt + j];
       if (st > 0) nsim = st * T.ndat / T.doms[slot].dtot;
       else use = false;  // dat::llh returns 0 for a DOM without simulated hits
     }
     if (use) v = llf(s, T.block_dat[b], nsim, T.ndat, T.sig, err);
   }
   if (err) atomicAdd(T.errors, 1);
-  const double total = cta_sum(v, sh);
-  if (threadIdx.x == 0) T.partial[(size_t)j * gridDim.x + blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kThreads) k_llh_final(const double* partial, int nparts,
-                                                        const unsigned long long* nohit, int norm, double nsim,
-                                                        double ndat, double sig, int ndof, int* errors, double* out) {
-  __shared__ double sh[kThreads];
-  const int j = blockIdx.x;
-  double v = 0;
-  for (int c = threadIdx.x; c < nparts; c += kThreads) v += partial[(size_t)j * nparts + c];
+  const double sum = cta_sum(v, sh);
+  // the last CTA of the shift to get here adds up the CTAs' sums (each of them written, and
+  // made visible, before its ticket)
+  if (threadIdx.x == 0) {
+    T.partial[(size_t)j * gridDim.x + blockIdx.x] = sum;
+    __threadfence();
+    last = atomicAdd(&T.ticket[j], 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  v = 0;
+  for (int c = threadIdx.x; c < gridDim.x; c += kThreads) v += __ldcg(&T.partial[(size_t)j * gridDim.x + c]);
   const double total = cta_sum(v, sh);
   if (threadIdx.x == 0) {
     double nh = 0;
-    bool err = false;
-    if (!norm) nh = llf((double)*nohit, 0, nsim, ndat, sig, err);
-    if (err) atomicAdd(errors, 1);
-    out[j] = (nh + total) / ndof;
+    err = false;
+    if (!T.norm) nh = llf((double)*T.nohit, 0, T.nsim, T.ndat, T.sig, err);
+    if (err) atomicAdd(T.errors, 1);
+    T.out[j] = (nh + total) / T.ndof;
   }
 }
 
@@ -201,6 +317,21 @@ T* upload_vec(const std::vector<T>& v, const char* what) {
   check(cudaMalloc((void**)&p, n * sizeof(T)), what);
   if (!v.empty()) check(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), what);
   return p;
+}
+
+// The counting kernels' shared-memory limit, once per device (a function attribute; before
+// any stream capture that launches them there).
+void count_prepare() {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  check(cudaGetDevice(&dev), "cudaGetDevice");
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load() & bit) return;
+  check(cudaFuncSetAttribute(k_llh_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem),
+        "likelihood attribute");
+  check(cudaFuncSetAttribute(k_llh_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem),
+        "likelihood attribute");
+  done.fetch_or(bit);
 }
 
 }  // namespace
@@ -220,7 +351,6 @@ void Likelihood::upload() {
   std::vector<double2> w(win.size() / 2);
   for (size_t k = 0; k < w.size(); k++) w[k] = make_double2(win[2 * k], win[2 * k + 1]);
   D.win = upload_vec(w, "likelihood tables");
-  check(cudaMalloc((void**)&D.nohit, sizeof(unsigned long long)), "likelihood scratch");
   check(cudaMalloc((void**)&D.errors, sizeof(int)), "likelihood scratch");
   check(cudaMemset(D.errors, 0, sizeof(int)), "likelihood scratch");
 }
@@ -242,63 +372,101 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   LlhDevice& D = *d_;
   const int nblocks = (int)blocks.size(), ndom = (int)doms.size();
   const int parts = std::max(1, (nblocks + kThreads - 1) / kThreads);
+  // the evaluation's counters: no-hit total, tickets, [block][shift], [DOM][shift] with norm
+  const size_t ntick = (ndt + 1) / 2 * 2, nsimc = ((size_t)ndt * nblocks + 1) / 2 * 2;
+  auto words = [&](int m) {
+    return 2 + (size_t)(m + 1) / 2 * 2 + ((size_t)m * nblocks + 1) / 2 * 2 + (opts.norm ? (size_t)m * ndom : 0);
+  };
   if (ndt > D.ndt_cap) {
-    for (void** p : {(void**)&D.simc, (void**)&D.stot, (void**)&D.partial})
+    for (void** p : {(void**)&D.work, (void**)&D.partial})
       if (*p) {
         cudaFree(*p);
         *p = nullptr;
       }
     D.ndt_cap = 0;
-    check(cudaMalloc((void**)&D.simc, (size_t)ndt * std::max(1, nblocks) * sizeof(unsigned int)), "likelihood scratch");
-    check(cudaMalloc((void**)&D.stot, (size_t)ndt * std::max(1, ndom) * sizeof(unsigned int)), "likelihood scratch");
+    check(cudaMalloc((void**)&D.work, words(ndt) * sizeof(unsigned int)), "likelihood scratch");
     check(cudaMalloc((void**)&D.partial, (size_t)ndt * parts * sizeof(double)), "likelihood scratch");
     D.ndt_cap = ndt;
   }
-  check(cudaMemsetAsync(D.simc, 0, (size_t)ndt * std::max(1, nblocks) * sizeof(unsigned int), st), "memset");
-  check(cudaMemsetAsync(D.stot, 0, (size_t)ndt * std::max(1, ndom) * sizeof(unsigned int), st), "memset");
-  check(cudaMemsetAsync(D.nohit, 0, sizeof(unsigned long long), st), "memset");
+  unsigned long long* nohit = reinterpret_cast<unsigned long long*>(D.work);
+  unsigned int* ticket = D.work + 2;
+  unsigned int* simc = ticket + ntick;
+  unsigned int* stot = simc + nsimc;
+  check(cudaMemsetAsync(D.work, 0, words(ndt) * sizeof(unsigned int), st), "memset");
   if (n > 0) {
-    const uint64_t grid = (n + kThreads - 1) / kThreads;
-    if (grid > 0x7fffffffull) throw Error("likelihood: too many hits in one call", 7);
-    FillArgs F;
+    if ((n + kThreads - 1) / kThreads > 0x7fffffffull) throw Error("likelihood: too many hits in one call", 7);
+    CountArgs F;
     F.A = back_args(eng_, dev_, dhits, n, seed);
     F.dom_slot = D.dom_slot;
     F.doms = D.doms;
     F.bin_block = D.bin_block;
     F.win = D.win;
-    F.simc = D.simc;
-    F.stot = D.stot;
-    F.nohit = D.nohit;
+    F.list = nullptr;
+    F.simc = simc;
+    F.stot = stot;
+    F.nohit = nohit;
     F.t0 = t0;
     F.lbin = lbin;
     F.nblocks = nblocks;
-    F.ndom = ndom;
     F.ndt = ndt;
     F.unh = opts.unh;
     F.norm = opts.norm;
     for (int j = 0; j < PPCB_LLH_MAX_SHIFTS; j++) F.dt[j] = j < ndt ? dts[j] : 0.0;
-    k_llh_fill<<<(unsigned int)grid, kThreads, 0, st>>>(F);
-    check(cudaGetLastError(), "likelihood fill");
+    // shifts per pass: as many as have their counters in shared memory; when not even one
+    // shift's fit, all of them in one pass over counters in global memory
+    const size_t row = (size_t)std::max(1, nblocks) * sizeof(unsigned int);
+    F.smem = row <= kCountSmem;
+    const int step = F.smem ? (int)std::min<size_t>(ndt, kCountSmem / row) : ndt;
+    const size_t smem = F.smem ? (size_t)step * row : 0;
+    count_prepare();
+    // a CTA per SM, fewer when there are less than 256 hits for each: every CTA clears and
+    // adds up counters of its own (3e4 hits, 64 shifts: 45 us with 2048 hits per CTA)
+    const uint64_t sms = eng_.devs.at(dev_).prop.multiProcessorCount;
+    const unsigned int grid = (unsigned int)std::max<uint64_t>(1, std::min<uint64_t>(sms, (n + 255) / 256));
+    // more than one pass: the acceptance once, into a list kept between calls (a captured
+    // call cannot grow it and accepts in every pass instead)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (step < ndt && n > D.list_cap) check(cudaStreamIsCapturing(st, &cap), "capture status");
+    if (step < ndt && (n <= D.list_cap || cap == cudaStreamCaptureStatusNone)) {
+      if (n > D.list_cap) {
+        if (D.list) cudaFree(D.list);
+        D.list = nullptr;
+        D.list_cap = 0;
+        check(cudaMalloc((void**)&D.list, n * sizeof(float2)), "likelihood scratch");
+        D.list_cap = n;
+      }
+      k_llh_accept<<<(unsigned int)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(F.A, D.dom_slot, D.list);
+      check(cudaGetLastError(), "likelihood acceptance");
+      F.list = D.list;
+    }
+    for (F.j0 = 0; F.j0 < ndt; F.j0 += step) {
+      F.nj = std::min(step, ndt - F.j0);
+      if (F.list) k_llh_count<true><<<grid, kCountThreads, smem, st>>>(F);
+      else k_llh_count<false><<<grid, kCountThreads, smem, st>>>(F);
+      check(cudaGetLastError(), "likelihood count");
+    }
   }
   TermArgs T;
-  T.simc = D.simc;
-  T.stot = D.stot;
+  T.simc = simc;
+  T.stot = stot;
+  T.nohit = nohit;
+  T.ticket = ticket;
   T.block_dat = D.block_dat;
   T.block_dom = D.block_dom;
   T.doms = D.doms;
   T.partial = D.partial;
   T.errors = D.errors;
+  T.out = dout;
   T.nsim = nsim;
   T.ndat = opts.drep;
   T.sig = opts.sig;
   T.nblocks = nblocks;
   T.ndom = ndom;
+  T.ndt = ndt;
   T.norm = opts.norm;
+  T.ndof = ndof;
   k_llh_terms<<<dim3(parts, ndt), kThreads, 0, st>>>(T);
   check(cudaGetLastError(), "likelihood terms");
-  k_llh_final<<<ndt, kThreads, 0, st>>>(D.partial, parts, D.nohit, opts.norm, nsim, opts.drep, opts.sig, ndof,
-                                        D.errors, dout);
-  check(cudaGetLastError(), "likelihood sum");
 }
 
 void Likelihood::require_device() {
