@@ -7,7 +7,7 @@
 //   bunching                            gpu/f2k.cxx:377-385 (addh)
 // Three kernels: k_src_count (one thread per source: its bunch template, the light
 // fluctuation and the Poisson count, from the source's own random stream; bunch and photon
-// totals per block of 256 sources), k_src_scan (offsets of the blocks), k_src_write (offsets
+// totals per block of 128 sources), k_src_scan (offsets of the blocks), k_src_write (offsets
 // within the block by a CTA scan; the bunches and their first-photon indices).  A source
 // makes ceil(count / 2^31) bunches.  This file is compiled without fast-math and without
 // contraction, so the bunch templates follow the host front end's float arithmetic.
@@ -23,21 +23,19 @@ namespace ppcb {
 
 struct FrontScratch {
   unsigned long long* num = nullptr;      // photons per source
-  unsigned long long* blk_rec = nullptr;  // bunches per block of kThreads sources
-  unsigned long long* blk_ph = nullptr;   // photons per block
-  unsigned long long* rec_off = nullptr;  // [blocks + 1] first bunch of each block
-  unsigned long long* ph_off = nullptr;   // [blocks + 1] first photon of each block
+  ulonglong2* tot = nullptr;              // bunches and photons per block of kThreads sources
+  ulonglong2* off = nullptr;              // [blocks + 1] first bunch and photon of each block
   int* errors = nullptr;
   uint64_t cap = 0;
   ~FrontScratch() {
-    for (void* p : {(void*)num, (void*)blk_rec, (void*)blk_ph, (void*)rec_off, (void*)ph_off, (void*)errors})
+    for (void* p : {(void*)num, (void*)tot, (void*)off, (void*)errors})
       if (p) cudaFree(p);
   }
 };
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;
 constexpr unsigned long long kMaxBunch = 1ull << 31;  // photons per bunch record
 constexpr int kMaxTries = 100000;                     // bound on every rejection loop
 constexpr float kRho = 0.9216f;                       // density of ice [mwe]
@@ -56,7 +54,7 @@ __device__ SrcRng src_stream(uint32_t seed, uint64_t k, const uint32_t* rm, uint
   z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
   z ^= z >> 31;
   SrcRng r;
-  r.a = rm[k % nmul];
+  r.a = __ldg(&rm[(nmul & (nmul - 1)) ? (uint32_t)(k % nmul) : (uint32_t)k & (nmul - 1)]);
   r.x = (uint32_t)z;
   r.y = __umulhi((uint32_t)(z >> 32), r.a);
   return r;
@@ -82,8 +80,32 @@ __device__ double src_gammln(double xx) {
   return -tmp + log(stp * ser);
 }
 
+// One proposal of the rejection sampler in the reference's double precision: the count
+// proposed by tan(x), or -1 when it is negative; its acceptance t in *t.
+__device__ __noinline__ double src_proposal(double xm, float x, double* t) {
+  const double sq = sqrt(2 * xm), alxm = log(xm), g = xm * alxm - src_gammln(xm + 1);
+  const double y = tan((double)x), em = sq * y + xm;
+  if (em < 0) return -1;
+  const double um = floor(em);
+  *t = 0.9 * (1 + y * y) * exp(um * alxm - src_gammln(um + 1) - g);
+  return um;
+}
+
 // Poisson sample of mean xm (gpu/f2k.cxx:402-433): multiplication of uniforms below 12,
-// rejection from a Lorentzian above
+// rejection from a Lorentzian above.  A proposal is first evaluated in single precision, with
+// bounds on its error: y = tan(x) to 4 units in the last place (7e-7 with its product by
+// sqrt(2 xm)), so the count floor(sqrt(2 xm) y + xm) is certain unless the sum lies that close
+// to an integer; and the logarithm of the Poisson ratio, by Stirling's series, as
+//   L = B - A + 1/(12 xm) - 1/(12 um),  A = (um + 1/2) log1p(B / xm),  B = um - xm,
+// to 7e-7 |A| + 1e-7 |B| + 1e-5 (the quotient's and the logarithm's roundings, the series' next
+// term for um >= 8).  Below means of 1e9 the double-precision sums round by less than that.
+// Where the count, or the comparison of the uniform number with the acceptance, is not certain,
+// src_proposal evaluates the reference's expressions (one proposal in 2e3 at a mean of 1000).
+// So the samples are those of the double-precision sampler, which spends 500 instructions on
+// a proposal (a double-precision tangent, exponential and six divisions) to 130 here.
+// Bound by issue and by lanes that wait for the unluckiest of their warp: the counts of 1e6
+// sources take 80 us instead of 157 (a thread that goes on to its next source while others
+// still reject: 95 us, the loop's state costs more than the waiting).
 __device__ unsigned long long src_poisson(double xm, SrcRng& r, bool& err) {
   if (isnan(xm)) {
     err = true;
@@ -103,18 +125,38 @@ __device__ unsigned long long src_poisson(double xm, SrcRng& r, bool& err) {
     }
     return um;
   }
-  const double sq = sqrt(2 * xm), alxm = log(xm), g = xm * alxm - src_gammln(xm + 1);
-  for (int it = 0; it < kMaxTries; it++) {
-    double y, em;
-    int k = 0;
-    do {
-      y = tan((double)(PPCB_FPI * r.u()));
-      em = sq * y + xm;
-    } while (em < 0 && ++k < kMaxTries);
-    if (em < 0) break;
-    const double um = floor(em);
-    const double t = 0.9 * (1 + y * y) * exp(um * alxm - src_gammln(um + 1) - g);
-    if (!(r.u() > t)) return (unsigned long long)um;
+  const float mf = (float)xm, sq = sqrtf(2 * mf), rx = 1 / mf;
+  int negative = 0;  // proposals below zero in a row
+  for (int it = 0; it < kMaxTries;) {
+    const float x = PPCB_FPI * r.u();
+    const float y = tanf(x), p = sq * y;
+    const double em = xm + (double)p;
+    double um = floor(em);
+    const float away = (float)(em - um);  // from the next integer below
+    const float slack = 1e-6f * fabsf(p) + 1e-6f;
+    double t = 0;
+    bool exact = !(away > slack && away < 1 - slack && (um >= 8 || em < 0) && xm < 1e9);
+    if (exact) um = src_proposal(xm, x, &t);
+    if (um < 0) {
+      if (++negative >= kMaxTries) break;
+      continue;
+    }
+    negative = 0;
+    it++;
+    const float u = r.u();
+    if (!exact) {
+      const float uf = (float)um, B = (float)(um - xm);
+      const float A = (uf + 0.5f) * log1pf(B * rx);
+      const float L = (B - A) + (rx - 1 / uf) * (1.f / 12);
+      const float margin = 1e-6f * fabsf(A) + 2e-7f * fabsf(B) + 3e-5f;
+      const float tf = 0.9f * (1 + y * y) * expf(L);
+      if (margin < 0.1f && u < tf * (1 - 2 * margin)) return (unsigned long long)um;
+      // a tiny ratio: exp(L) is below the smallest uniform number, whatever its error
+      if ((margin < 0.1f && u > tf * (1 + 2 * margin)) || (L + 1.001f * logf(1 + y * y) < -20 - 2 * margin)) continue;
+      um = src_proposal(xm, x, &t);
+      if (um < 0) continue;
+    }
+    if (!(u > t)) return (unsigned long long)um;
   }
   err = true;
   return (unsigned long long)floor(xm + 0.5);
@@ -249,8 +291,7 @@ struct SrcArgs {
   uint32_t nmul, seed;
   float eff, ovr;
   unsigned long long* num;
-  unsigned long long* blk_rec;
-  unsigned long long* blk_ph;
+  ulonglong2* tot;
   int* errors;
 };
 
@@ -292,11 +333,30 @@ __device__ __forceinline__ unsigned long long src_bunches(unsigned long long num
   return (num + kMaxBunch - 1) / kMaxBunch;
 }
 
+constexpr unsigned int kSrcWords = sizeof(ppcb_source) / 4;
+
+// Copies n 4-byte words from global to shared memory, 16 bytes at a time where the global
+// address allows it.
+__device__ __forceinline__ void copy_words(uint32_t* dst, const uint32_t* src, unsigned int n) {
+  unsigned int done = 0;
+  if (reinterpret_cast<uintptr_t>(src) % 16 == 0) {
+    const unsigned int q = n / 4;
+    for (unsigned int i = threadIdx.x; i < q; i += kThreads)
+      reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    done = 4 * q;
+  }
+  for (unsigned int i = done + threadIdx.x; i < n; i += kThreads) dst[i] = src[i];
+}
+
 __global__ void __launch_bounds__(kThreads) k_src_count(SrcArgs A) {
-  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+  __shared__ __align__(16) uint32_t in[kThreads * kSrcWords];
+  const uint64_t k0 = (uint64_t)blockIdx.x * kThreads, k = k0 + threadIdx.x;
+  copy_words(in, reinterpret_cast<const uint32_t*>(A.src + k0),
+             (unsigned int)min((uint64_t)kThreads, A.n - k0) * kSrcWords);
+  __syncthreads();
   unsigned long long num = 0;
   if (k < A.n) {
-    const ppcb_source s = A.src[k];
+    const ppcb_source& s = reinterpret_cast<const ppcb_source*>(in)[threadIdx.x];
     SrcRng r = src_stream(A.seed, k, A.rm, A.nmul);
     ppcb_bunch p;
     bool err = false;
@@ -312,75 +372,133 @@ __global__ void __launch_bounds__(kThreads) k_src_count(SrcArgs A) {
   }
   unsigned long long nr = src_bunches(num), np = num, tr, tp;
   cta_scan2(nr, np, &tr, &tp);
-  if (threadIdx.x == 0) {
-    A.blk_rec[blockIdx.x] = tr;
-    A.blk_ph[blockIdx.x] = tp;
-  }
+  if (threadIdx.x == 0) A.tot[blockIdx.x] = make_ulonglong2(tr, tp);
 }
 
-// exclusive scans of the blocks' bunch and photon totals (one block, a contiguous chunk of
-// blocks per thread)
-__global__ void k_src_scan(const unsigned long long* nrec, const unsigned long long* num, uint64_t n,
-                           unsigned long long* rec_off, unsigned long long* ph_off, uint64_t* counts) {
-  __shared__ unsigned long long pr[1024], pp[1024];
-  const uint64_t t = threadIdx.x, nt = blockDim.x;
-  const uint64_t per = (n + nt - 1) / nt;
-  const uint64_t lo = min(n, t * per), hi = min(n, lo + per);
-  unsigned long long sr = 0, sp = 0;
-  for (uint64_t k = lo; k < hi; k++) {
-    sr += nrec[k];
-    sp += num[k];
-  }
-  pr[t] = sr;
-  pp[t] = sp;
-  __syncthreads();
-  for (unsigned int d = 1; d < nt; d <<= 1) {
-    const unsigned long long vr = t >= d ? pr[t - d] : 0, vp = t >= d ? pp[t - d] : 0;
+// Exclusive scans of the blocks' bunch and photon totals (one block, kChunk blocks of sources
+// per thread and turn).
+constexpr int kScanThreads = 1024, kChunk = 4;
+static_assert(kScanThreads == 32 * 32, "one warp scans the warps' totals");
+__global__ void __launch_bounds__(kScanThreads) k_src_scan(const ulonglong2* tot, uint64_t n, ulonglong2* off,
+                                                           uint64_t* counts) {
+  __shared__ unsigned long long wr[kScanThreads / 32], wp[kScanThreads / 32];
+  const unsigned int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long br = 0, bp = 0;
+  for (uint64_t t0 = 0; t0 < n; t0 += kChunk * kScanThreads) {
+    const uint64_t t = t0 + kChunk * threadIdx.x;
+    ulonglong2 c[kChunk];
+    unsigned long long sr = 0, sp = 0;
+#pragma unroll
+    for (int q = 0; q < kChunk; q++) {
+      c[q] = t + q < n ? tot[t + q] : make_ulonglong2(0, 0);
+      sr += c[q].x;
+      sp += c[q].y;
+    }
+    unsigned long long ur = sr, up = sp;
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long xr = __shfl_up_sync(0xffffffffu, ur, d), xp = __shfl_up_sync(0xffffffffu, up, d);
+      if ((int)lane >= d) {
+        ur += xr;
+        up += xp;
+      }
+    }
+    if (lane == 31) {
+      wr[w] = ur;
+      wp[w] = up;
+    }
     __syncthreads();
-    pr[t] += vr;
-    pp[t] += vp;
+    ur += br - sr;
+    up += bp - sp;
+    if (w == 0) {  // the warps' totals
+      unsigned long long r = wr[lane], p = wp[lane];
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long xr = __shfl_up_sync(0xffffffffu, r, d), xp = __shfl_up_sync(0xffffffffu, p, d);
+        if ((int)lane >= d) {
+          r += xr;
+          p += xp;
+        }
+      }
+      wr[lane] = r;
+      wp[lane] = p;
+    }
     __syncthreads();
-  }
-  unsigned long long ar = pr[t] - sr, ap = pp[t] - sp;
-  for (uint64_t k = lo; k < hi; k++) {
-    rec_off[k] = ar;
-    ph_off[k] = ap;
-    ar += nrec[k];
-    ap += num[k];
-  }
-  if (t == nt - 1) {
-    rec_off[n] = pr[t];
-    ph_off[n] = pp[t];
-    counts[0] = pr[t];
-    counts[1] = pp[t];
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_src_write(SrcArgs A, const unsigned long long* rec_off,
-                                                        const unsigned long long* ph_off, uint64_t nblk,
-                                                        ppcb_bunch* out, uint64_t* bstart, uint64_t cap) {
-  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  const unsigned long long num = k < A.n ? A.num[k] : 0, nrec = src_bunches(num);
-  unsigned long long b0 = nrec, ph0 = num, tr, tp;
-  cta_scan2(b0, ph0, &tr, &tp);
-  if (k >= A.n) return;
-  b0 += rec_off[blockIdx.x];
-  ph0 += ph_off[blockIdx.x];
-  if (nrec > 0) {
-    const ppcb_source s = A.src[k];
-    ppcb_bunch p;
-    bool err = false;
-    src_bunch(s, A.eff, A.ovr, p, nullptr, err);
-    for (unsigned long long j = 0; j < nrec; j++) {
-      const unsigned long long b = b0 + j;
-      if (b >= cap) break;
-      const unsigned long long left = num - j * kMaxBunch;
-      p.num = (uint32_t)(left < kMaxBunch ? left : kMaxBunch);
-      out[b] = p;
-      bstart[b] = ph0 + j * kMaxBunch;
+    if (w > 0) {
+      ur += wr[w - 1];
+      up += wp[w - 1];
+    }
+    br += wr[31];
+    bp += wp[31];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kChunk; q++) {
+      if (t + q < n) off[t + q] = make_ulonglong2(ur, up);
+      ur += c[q].x;
+      up += c[q].y;
     }
   }
-  if (k == A.n - 1 && rec_off[nblk] <= cap) bstart[rec_off[nblk]] = ph_off[nblk];
+  if (threadIdx.x == 0) {
+    off[n] = make_ulonglong2(br, bp);
+    counts[0] = br;
+    counts[1] = bp;
+  }
+}
+
+// Where the 16-byte word e of the staged bunches lies: records four words apart, written by
+// eight threads at a time, then fall on eight different banks.
+__device__ __forceinline__ unsigned int swizzle(unsigned int e) { return e ^ ((e >> 3) & 7); }
+
+// The block's sources come in, and its bunches go out, as coalesced runs through shared memory
+// (a thread's own 72-byte loads and 64-byte stores touch a sector or two each: 77 us for 1e6
+// sources, 36 us this way, 24 us at the memory's rate).  A block with a source of several bunches (2^31 photons and
+// more) or at the end of the caller's buffer writes its records one by one.
+__global__ void __launch_bounds__(kThreads) k_src_write(SrcArgs A, const ulonglong2* off, uint64_t nblk,
+                                                        ppcb_bunch* out, uint64_t* bstart, uint64_t cap) {
+  __shared__ __align__(16) uint32_t in[kThreads * kSrcWords];
+  __shared__ uint4 stage[kThreads * 4];
+  static_assert(sizeof(ppcb_bunch) == 4 * sizeof(uint4), "a bunch is four 16-byte words");
+  const uint64_t k0 = (uint64_t)blockIdx.x * kThreads, k = k0 + threadIdx.x;
+  const unsigned int mine = (unsigned int)min((uint64_t)kThreads, A.n - k0);
+  copy_words(in, reinterpret_cast<const uint32_t*>(A.src + k0), mine * kSrcWords);
+  const unsigned long long num = k < A.n ? A.num[k] : 0, nrec = src_bunches(num);
+  unsigned long long b0 = nrec, ph0 = num, tr, tp;
+  cta_scan2(b0, ph0, &tr, &tp);  // a barrier: `in` is complete
+  const ulonglong2 o = off[blockIdx.x];
+  const bool run = tr <= kThreads && o.x + tr <= cap && !__syncthreads_or(nrec > 1);
+  if (nrec > 0) {
+    const ppcb_source& s = reinterpret_cast<const ppcb_source*>(in)[threadIdx.x];
+    __align__(16) ppcb_bunch p;
+    bool err = false;
+    src_bunch(s, A.eff, A.ovr, p, nullptr, err);
+    if (run) {
+      p.num = (uint32_t)num;
+      const uint4* w = reinterpret_cast<const uint4*>(&p);
+#pragma unroll
+      for (unsigned int q = 0; q < 4; q++) stage[swizzle(4 * (unsigned int)b0 + q)] = w[q];
+      bstart[o.x + b0] = o.y + ph0;
+    } else {
+      for (unsigned long long j = 0; j < nrec; j++) {
+        const unsigned long long b = o.x + b0 + j;
+        if (b >= cap) break;
+        const unsigned long long left = num - j * kMaxBunch;
+        p.num = (uint32_t)(left < kMaxBunch ? left : kMaxBunch);
+        out[b] = p;
+        bstart[b] = o.y + ph0 + j * kMaxBunch;
+      }
+    }
+  }
+  if (run) {
+    __syncthreads();
+    const unsigned int n = 4 * (unsigned int)tr;
+    if (reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+      uint4* dst = reinterpret_cast<uint4*>(out + o.x);
+      for (unsigned int e = threadIdx.x; e < n; e += kThreads) dst[e] = stage[swizzle(e)];
+    } else {  // the caller's records need only their own 4-byte alignment
+      uint32_t* dst = reinterpret_cast<uint32_t*>(out + o.x);
+      for (unsigned int i = threadIdx.x; i < 4 * n; i += kThreads)
+        dst[i] = reinterpret_cast<const uint32_t*>(&stage[swizzle(i / 4)])[i % 4];
+    }
+  }
+  if (k == A.n - 1 && off[nblk].x <= cap) bstart[off[nblk].x] = off[nblk].y;
 }
 
 }  // namespace
@@ -404,17 +522,15 @@ void Engine::sources(int d, const ppcb_source* dsrc, uint64_t ns, uint32_t seed,
   }
   FrontScratch& F = *g.front;
   if (ns > F.cap) {
-    for (void** p : {(void**)&F.num, (void**)&F.blk_rec, (void**)&F.blk_ph, (void**)&F.rec_off, (void**)&F.ph_off})
+    for (void** p : {(void**)&F.num, (void**)&F.tot, (void**)&F.off})
       if (*p) {
         cudaFree(*p);
         *p = nullptr;
       }
     F.cap = 0;
     check(cudaMalloc((void**)&F.num, ns * sizeof(unsigned long long)), "front end scratch");
-    check(cudaMalloc((void**)&F.blk_rec, grid * sizeof(unsigned long long)), "front end scratch");
-    check(cudaMalloc((void**)&F.blk_ph, grid * sizeof(unsigned long long)), "front end scratch");
-    check(cudaMalloc((void**)&F.rec_off, (grid + 1) * sizeof(unsigned long long)), "front end scratch");
-    check(cudaMalloc((void**)&F.ph_off, (grid + 1) * sizeof(unsigned long long)), "front end scratch");
+    check(cudaMalloc((void**)&F.tot, grid * sizeof(ulonglong2)), "front end scratch");
+    check(cudaMalloc((void**)&F.off, (grid + 1) * sizeof(ulonglong2)), "front end scratch");
     F.cap = ns;
   }
   SrcArgs A;
@@ -426,14 +542,13 @@ void Engine::sources(int d, const ppcb_source* dsrc, uint64_t ns, uint32_t seed,
   A.eff = cfg.eff;
   A.ovr = cfg.ovr;
   A.num = F.num;
-  A.blk_rec = F.blk_rec;
-  A.blk_ph = F.blk_ph;
+  A.tot = F.tot;
   A.errors = F.errors;
   k_src_count<<<(unsigned int)grid, kThreads, 0, st>>>(A);
   check(cudaGetLastError(), "front end count");
-  k_src_scan<<<1, 1024, 0, st>>>(F.blk_rec, F.blk_ph, grid, F.rec_off, F.ph_off, dcounts);
+  k_src_scan<<<1, kScanThreads, 0, st>>>(F.tot, grid, F.off, dcounts);
   check(cudaGetLastError(), "front end scan");
-  k_src_write<<<(unsigned int)grid, kThreads, 0, st>>>(A, F.rec_off, F.ph_off, grid, dout, dbstart, cap);
+  k_src_write<<<(unsigned int)grid, kThreads, 0, st>>>(A, F.off, grid, dout, dbstart, cap);
   check(cudaGetLastError(), "front end write");
 }
 
