@@ -1280,7 +1280,7 @@ __device__ __forceinline__ long long charge_bin(const ppcb_hit& h, uint32_t even
 // the path's per-layer derivative terms, weighted by the hit's DOM weight, until the
 // recorded hit is reached again.  A replay that does not end on the recorded hit (same
 // DOM, same time bits) is counted in stats[1].
-__global__ void __launch_bounds__(256, 3) k_adjoint(const __grid_constant__ KArgs a, const ppcb_hit* __restrict__ hits,
+__global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_constant__ KArgs a, const ppcb_hit* __restrict__ hits,
                                                  const Prov* __restrict__ prov, uint64_t cap,
                                                  const unsigned long long* nh_dev, uint32_t events,
                                                  const float* __restrict__ wdom, const float2* __restrict__ wgrad,
@@ -1294,7 +1294,10 @@ __global__ void __launch_bounds__(256, 3) k_adjoint(const __grid_constant__ KArg
   load_tables(a, S);
   const DynTabs dt = load_dyn(a, dsm);
   unsigned int nan_steps = 0, replayed = 0, unmatched = 0;
-  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < nh; k += (uint64_t)gridDim.x * blockDim.x) {
+  // consecutive hits go to different blocks: a replay of few hits is bound by the latency of
+  // its longest path, which is shorter on an SM that has few of them (417 hits with their
+  // histogram and weights 0.64 -> 0.47 ms, 85 000 hits 1.20 -> 1.18 ms)
+  for (uint64_t k = blockIdx.x + threadIdx.x * (uint64_t)gridDim.x; k < nh; k += (uint64_t)gridDim.x * blockDim.x) {
     const ppcb_hit h = hits[k];
     const long long bin = charge_bin(h, events, a.p.gsize);
     const float w = bin >= 0 ? wdom[bin] : 0.f;

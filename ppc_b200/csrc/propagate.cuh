@@ -74,6 +74,7 @@ cudaError_t launch_adjoint(const KArgs& a, const ppcb_hit* hits, const void* pro
                            cudaStream_t st, const unsigned long long* nh_dev = nullptr);
 cudaError_t launch_dom_hist(const ppcb_hit* hits, uint64_t nh, unsigned int* counts, uint32_t events, int gsize,
                             cudaStream_t st, const unsigned long long* nh_dev = nullptr);
+constexpr int kAdjointPerSm = 3;  // resident blocks of the replay per SM
 cudaError_t adjoint_prepare();  // the replay's launch attribute on the current device (before a capture)
 constexpr size_t kProvBytes = 64;  // provenance record per hit slot of the gradient's recording pass
 cudaError_t propagate_attributes(int* regs, int* max_threads, size_t* smem, size_t* local);
