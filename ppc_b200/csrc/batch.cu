@@ -67,6 +67,7 @@ Batch::Batch(Engine& e, int device, uint32_t max_events, uint32_t max_bunches, u
   check(cudaSetDevice(cuda_dev_), "cudaSetDevice");
   check(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking), "stream");
   for (cudaEvent_t* ev : {&k0_, &k1_, &g0_, &g1_}) check(cudaEventCreate(ev), "event");
+  check(cudaEventCreateWithFlags(&end_, cudaEventDisableTiming), "event");
   bunches_ = dmalloc<ppcb_bunch>(maxB_);
   bstart_ = dmalloc<uint64_t>(maxB_ + 1);
   ev_off_ = dmalloc<uint64_t>(maxE_);
@@ -100,7 +101,7 @@ Batch::~Batch() {
   for (void* p : d) if (p) cudaFree(p);
   void* h[] = {h_bunches_, h_bstart_, h_ev_off_, h_ev_cap_, h_ev_cnt_, h_dyn_, h_out_off_, h_ctrl_};
   for (void* p : h) if (p) cudaFreeHost(p);
-  for (cudaEvent_t ev : {k0_, k1_, g0_, g1_}) if (ev) cudaEventDestroy(ev);
+  for (cudaEvent_t ev : {k0_, k1_, g0_, g1_, end_}) if (ev) cudaEventDestroy(ev);
   if (st_) cudaStreamDestroy(st_);
 }
 
@@ -195,7 +196,7 @@ void Batch::run(const ppcb_bunch* b, int nb, uint32_t events, BatchResult& out, 
             out_off_, ctrl_, h_bunches_, h_bstart_, h_ev_off_, h_ev_cap_, h_dyn_, h_ev_cnt_, h_out_off_, h_ctrl_, g0_,
             k0_, k1_, g1_);
   }
-  check(cudaStreamSynchronize(st_), "batch");
+  wait_launch(st_, end_, num, "batch");
   out.produced.assign(h_ev_cnt_, h_ev_cnt_ + events);
   out.offset.assign(h_out_off_, h_out_off_ + events + 1);
   out.overflowed = 0;

@@ -51,7 +51,7 @@ class Batch {
   uint64_t hcap_;
   cudaStream_t st_ = nullptr;
   cudaGraphExec_t exec_ = nullptr;
-  cudaEvent_t k0_ = nullptr, k1_ = nullptr, g0_ = nullptr, g1_ = nullptr;
+  cudaEvent_t k0_ = nullptr, k1_ = nullptr, g0_ = nullptr, g1_ = nullptr, end_ = nullptr;
   // device
   ppcb_bunch* bunches_ = nullptr;
   uint64_t* bstart_ = nullptr;

@@ -212,30 +212,33 @@ int ppcb_accept(ppcb_ctx* c, const ppcb_hit* hits, uint64_t n, uint32_t seed, pp
     ppcb::Engine& e = c->s.eng;
     if (!e.ready()) throw ppcb::Error("ppcb_ini() must come before the back end", PPCB_ESTATE);
     ppcb::check(cudaSetDevice(e.devs[0].dev), "cudaSetDevice");
-    ppcb_hit* dh = nullptr;
-    ppcb_acc_hit* dout = nullptr;
-    unsigned long long* dcnt = nullptr;
-    auto release = [&]() {
-      if (dh) cudaFree(dh);
-      if (dout) cudaFree(dout);
-      if (dcnt) cudaFree(dcnt);
-    };
-    try {
-      ppcb::check(cudaMalloc((void**)&dh, std::max<uint64_t>(n, 1) * sizeof(ppcb_hit)), "back end input");
-      ppcb::check(cudaMalloc((void**)&dout, std::max<uint64_t>(n, 1) * sizeof(ppcb_acc_hit)), "back end output");
-      ppcb::check(cudaMalloc((void**)&dcnt, sizeof(unsigned long long)), "back end count");
-      if (n) ppcb::check(cudaMemcpy(dh, hits, n * sizeof(ppcb_hit), cudaMemcpyHostToDevice), "H2D hits");
-      e.accept(0, dh, n, seed, dout, dcnt, 0);
-      unsigned long long k = 0;
-      ppcb::check(cudaMemcpy(&k, dcnt, sizeof(k), cudaMemcpyDeviceToHost), "D2H count");
+    const std::shared_ptr<ppcb::CallBuffers> io = e.devs[0].io;
+    const ppcb::CallBuffers::Use use(*io);
+    const size_t in = n * sizeof(ppcb_hit), res = n * sizeof(ppcb_acc_hit), cnt = sizeof(unsigned long long);
+    ppcb_hit* dh = static_cast<ppcb_hit*>(io->device(0, in));
+    // the records, then (on its 8-byte boundary) their number
+    unsigned char* dout = static_cast<unsigned char*>(io->device(1, res + cnt));
+    unsigned char* h = io->stage(in + res + cnt);
+    unsigned long long k = 0;
+    if (h) {  // a small call: staged both ways, one wait; the records come back uncounted
+      if (n) std::memcpy(h, hits, in);
+      if (n) ppcb::check(cudaMemcpyAsync(dh, h, in, cudaMemcpyHostToDevice, 0), "H2D hits");
+      e.accept(0, dh, n, seed, reinterpret_cast<ppcb_acc_hit*>(dout), reinterpret_cast<unsigned long long*>(dout + res),
+               0);
+      ppcb::check(cudaMemcpyAsync(h + in, dout, res + cnt, cudaMemcpyDeviceToHost, 0), "D2H hits");
+      io->wait(0);
+      std::memcpy(&k, h + in + res, cnt);
+      const uint64_t w = std::min<uint64_t>(k, cap);
+      if (w && out) std::memcpy(out, h + in, w * sizeof(ppcb_acc_hit));
+    } else {
+      ppcb::check(cudaMemcpy(dh, hits, in, cudaMemcpyHostToDevice), "H2D hits");
+      e.accept(0, dh, n, seed, reinterpret_cast<ppcb_acc_hit*>(dout), reinterpret_cast<unsigned long long*>(dout + res),
+               0);
+      ppcb::check(cudaMemcpy(&k, dout + res, cnt, cudaMemcpyDeviceToHost), "D2H count");
       const uint64_t w = std::min<uint64_t>(k, cap);
       if (w && out) ppcb::check(cudaMemcpy(out, dout, w * sizeof(ppcb_acc_hit), cudaMemcpyDeviceToHost), "D2H");
-      *nout = k;
-    } catch (...) {
-      release();
-      throw;
     }
-    release();
+    *nout = k;
   });
 }
 
@@ -265,38 +268,52 @@ int ppcb_sources(ppcb_ctx* c, const ppcb_source* src, uint64_t ns, uint32_t seed
     ppcb::Engine& e = c->s.eng;
     if (!e.ready()) throw ppcb::Error("ppcb_ini() must come before the front end", PPCB_ESTATE);
     ppcb::check(cudaSetDevice(e.devs[0].dev), "cudaSetDevice");
-    const int before = e.front_errors(0);
-    ppcb_source* ds = nullptr;
-    ppcb_bunch* dout = nullptr;
-    uint64_t* dbs = nullptr;
-    uint64_t* dcnt = nullptr;
-    auto release = [&]() {
-      for (void* p : {(void*)ds, (void*)dout, (void*)dbs, (void*)dcnt})
-        if (p) cudaFree(p);
+    const std::shared_ptr<ppcb::CallBuffers> io = e.devs[0].io;
+    const ppcb::CallBuffers::Use use(*io);
+    const size_t in = ns * sizeof(ppcb_source), res = cap * sizeof(ppcb_bunch), off = (cap + 1) * sizeof(uint64_t);
+    ppcb_source* ds = static_cast<ppcb_source*>(io->device(0, in));
+    ppcb_bunch* dout = static_cast<ppcb_bunch*>(io->device(1, res));
+    uint64_t* dbs = static_cast<uint64_t*>(io->device(2, off));
+    uint64_t* dcnt = static_cast<uint64_t*>(io->device(3, 2 * sizeof(uint64_t)));
+    // staging: counts and the error counter before and after, then (in a small call, which
+    // waits once and brings the records back uncounted) the sources, records and offsets
+    unsigned char* h = io->stage(64 + in + res + off);
+    const bool small = h != nullptr;
+    if (!small) h = io->stage(64);
+    uint64_t* cnt = reinterpret_cast<uint64_t*>(h);
+    int* err = reinterpret_cast<int*>(h + 16);
+    err[0] = err[1] = 0;
+    auto fetch = [&](void* to, const void* from, size_t bytes, const char* what) {
+      if (bytes) ppcb::check(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, 0), what);
     };
-    try {
-      ppcb::check(cudaMalloc((void**)&ds, std::max<uint64_t>(ns, 1) * sizeof(ppcb_source)), "front end input");
-      ppcb::check(cudaMalloc((void**)&dout, std::max<uint64_t>(cap, 1) * sizeof(ppcb_bunch)), "front end output");
-      ppcb::check(cudaMalloc((void**)&dbs, (cap + 1) * sizeof(uint64_t)), "front end output");
-      ppcb::check(cudaMalloc((void**)&dcnt, 2 * sizeof(uint64_t)), "front end counts");
-      if (ns) ppcb::check(cudaMemcpy(ds, src, ns * sizeof(ppcb_source), cudaMemcpyHostToDevice), "H2D sources");
-      e.sources(0, ds, ns, seed, dout, dbs, cap, dcnt, 0);
-      uint64_t cnt[2];
-      ppcb::check(cudaMemcpy(cnt, dcnt, sizeof(cnt), cudaMemcpyDeviceToHost), "D2H counts");
-      const uint64_t w = std::min<uint64_t>(cnt[0], cap);
-      if (w) ppcb::check(cudaMemcpy(out, dout, w * sizeof(ppcb_bunch), cudaMemcpyDeviceToHost), "D2H bunches");
-      if (cap > 0 || cnt[0] == 0)
-        if (bstart)
-          ppcb::check(cudaMemcpy(bstart, dbs, (w + (cnt[0] <= cap ? 1 : 0)) * sizeof(uint64_t),
-                                 cudaMemcpyDeviceToHost), "D2H bunch starts");
-      *nb = cnt[0];
-      *num = cnt[1];
-    } catch (...) {
-      release();
-      throw;
+    if (const int* p = e.front_errors(0)) fetch(&err[0], p, sizeof(int), "D2H errors");
+    if (small) {
+      if (ns) std::memcpy(h + 64, src, in);
+      if (ns) ppcb::check(cudaMemcpyAsync(ds, h + 64, in, cudaMemcpyHostToDevice, 0), "H2D sources");
+    } else if (ns) {
+      ppcb::check(cudaMemcpy(ds, src, in, cudaMemcpyHostToDevice), "H2D sources");
     }
-    release();
-    if (e.front_errors(0) != before)
+    e.sources(0, ds, ns, seed, dout, dbs, cap, dcnt, 0);
+    fetch(cnt, dcnt, 2 * sizeof(uint64_t), "D2H counts");
+    if (const int* p = e.front_errors(0)) fetch(&err[1], p, sizeof(int), "D2H errors");
+    if (small) {
+      fetch(h + 64 + in, dout, res, "D2H bunches");
+      fetch(h + 64 + in + res, dbs, off, "D2H bunch starts");
+    }
+    io->wait(0);
+    const uint64_t w = std::min<uint64_t>(cnt[0], cap);
+    const size_t starts = (w + (cnt[0] <= cap ? 1 : 0)) * sizeof(uint64_t);
+    const bool want = bstart && (cap > 0 || cnt[0] == 0);
+    if (small) {
+      if (w) std::memcpy(out, h + 64 + in, w * sizeof(ppcb_bunch));
+      if (want) std::memcpy(bstart, h + 64 + in + res, starts);
+    } else {
+      if (w) ppcb::check(cudaMemcpy(out, dout, w * sizeof(ppcb_bunch), cudaMemcpyDeviceToHost), "D2H bunches");
+      if (want) ppcb::check(cudaMemcpy(bstart, dbs, starts, cudaMemcpyDeviceToHost), "D2H bunch starts");
+    }
+    *nb = cnt[0];
+    *num = cnt[1];
+    if (err[0] != err[1])
       throw ppcb::Error("front end: a source's sampling failed (negative type, bad count or no convergence)",
                         PPCB_EARG);
   });

@@ -2,6 +2,7 @@
 // likelihood on the device").
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <exception>
 #include <string>
 
@@ -102,25 +103,30 @@ int ppcb_llh_eval(ppcb_llh* l, const ppcb_hit* hits, uint64_t n, uint32_t seed, 
     ppcb::Likelihood& L = *l->l;
     if (ndt < 1 || ndt > PPCB_LLH_MAX_SHIFTS) throw ppcb::Error("likelihood: 1 to 64 time shifts per evaluation", 7);
     L.require_device();
-    const int before = L.errors();
-    ppcb_hit* dh = nullptr;
-    double* dout = nullptr;
-    auto release = [&]() {
-      if (dh) cudaFree(dh);
-      if (dout) cudaFree(dout);
-    };
-    try {
-      ppcb::check(cudaMalloc((void**)&dh, std::max<uint64_t>(n, 1) * sizeof(ppcb_hit)), "likelihood input");
-      ppcb::check(cudaMalloc((void**)&dout, ndt * sizeof(double)), "likelihood output");
-      if (n) ppcb::check(cudaMemcpy(dh, hits, n * sizeof(ppcb_hit), cudaMemcpyHostToDevice), "H2D hits");
-      L.eval_device(dh, n, seed, dts, ndt, nsim, dout, 0);
-      ppcb::check(cudaMemcpy(out, dout, ndt * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
-    } catch (...) {
-      release();
-      throw;
+    ppcb::CallBuffers& io = L.io();
+    const ppcb::CallBuffers::Use use(io);
+    const int* derr = L.device_errors();
+    const size_t in = n * sizeof(ppcb_hit), res = ndt * sizeof(double);
+    ppcb_hit* dh = static_cast<ppcb_hit*>(io.device(0, in));
+    double* dout = static_cast<double*>(io.device(1, res));
+    // staging: the error counter before and after, the results, and a small call's hits
+    unsigned char* h = io.stage(16 + res + in);
+    const bool small = h != nullptr;
+    if (!small) h = io.stage(16 + res);
+    int* err = reinterpret_cast<int*>(h);
+    ppcb::check(cudaMemcpyAsync(&err[0], derr, sizeof(int), cudaMemcpyDeviceToHost, 0), "D2H errors");
+    if (small && n) {
+      std::memcpy(h + 16 + res, hits, in);
+      ppcb::check(cudaMemcpyAsync(dh, h + 16 + res, in, cudaMemcpyHostToDevice, 0), "H2D hits");
+    } else if (n) {
+      ppcb::check(cudaMemcpy(dh, hits, in, cudaMemcpyHostToDevice), "H2D hits");
     }
-    release();
-    if (L.errors() != before)
+    L.eval_device(dh, n, seed, dts, ndt, nsim, dout, 0);
+    ppcb::check(cudaMemcpyAsync(h + 16, dout, res, cudaMemcpyDeviceToHost, 0), "D2H");
+    ppcb::check(cudaMemcpyAsync(&err[1], derr, sizeof(int), cudaMemcpyDeviceToHost, 0), "D2H errors");
+    io.wait(0);
+    std::memcpy(out, h + 16, res);
+    if (err[0] != err[1])
       throw ppcb::Error("llf: the Newton iteration left its domain (llh/llh.cxx:649-650)", PPCB_ECONFIG);
   });
 }

@@ -29,6 +29,56 @@ static void upload(T* d, const T* h, size_t n, const char* what) {
   if (n) check(cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice), what);
 }
 
+void wait_launch(cudaStream_t st, cudaEvent_t e, uint64_t photons, const char* what) {
+  check(cudaEventRecord(e, st), what);
+  check(photons <= kSpinPhotons ? cudaEventSynchronize(e) : cudaStreamSynchronize(st), what);
+}
+
+void* CallBuffers::device(int part, size_t bytes) {
+  bytes = std::max<size_t>(bytes, 16);
+  if (bytes > cap_[part]) {
+    if (dev_[part]) cudaFree(dev_[part]);
+    dev_[part] = nullptr;
+    cap_[part] = 0;
+    check(cudaMalloc(&dev_[part], bytes), "call buffer");
+    cap_[part] = bytes;
+  }
+  return dev_[part];
+}
+
+unsigned char* CallBuffers::stage(size_t bytes) {
+  if (bytes > kStageBytes) return nullptr;
+  if (bytes > pin_cap_) {
+    if (pin_) cudaFreeHost(pin_);
+    pin_ = nullptr;
+    pin_cap_ = 0;
+    check(cudaMallocHost(&pin_, bytes), "pinned call buffer");
+    pin_cap_ = bytes;
+  }
+  return static_cast<unsigned char*>(pin_);
+}
+
+void CallBuffers::trim() {
+  for (int k = 0; k < 4; k++)
+    if (cap_[k] > kKeepBytes) {
+      cudaFree(dev_[k]);
+      dev_[k] = nullptr;
+      cap_[k] = 0;
+    }
+}
+
+CallBuffers::~CallBuffers() {
+  for (void* p : dev_) if (p) cudaFree(p);
+  if (pin_) cudaFreeHost(pin_);
+  if (done_) cudaEventDestroy(done_);
+}
+
+void CallBuffers::wait(cudaStream_t st) {
+  if (!done_) check(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming), "event");
+  check(cudaEventRecord(done_, st), "event");
+  check(cudaEventSynchronize(done_), "call");
+}
+
 Engine::~Engine() {
   try { fin(); } catch (...) {}
 }
@@ -112,6 +162,7 @@ void Engine::ini() {
     pmax += pm;
     if (pmxo == 0 || pmxo > po) pmxo = po;
 
+    g.io = std::make_shared<CallBuffers>();
     check(cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking), "stream");
     check(cudaStreamCreateWithFlags(&g.cp, cudaStreamNonBlocking), "stream");
     const ppcb_params& p = cfg.p;
@@ -155,6 +206,7 @@ void Engine::ini() {
       check(cudaMallocHost((void**)&S.hb, g.bcap * sizeof(ppcb_bunch)), "pinned bunches");
       check(cudaMallocHost((void**)&S.hbstart, (g.bcap + 1) * sizeof(uint64_t)), "pinned bstart");
       check(cudaMallocHost((void**)&S.hctrl, sizeof(ppcb_ctrl)), "pinned ctrl");
+      check(cudaMallocHost((void**)&S.hfirst, kFirstHits * sizeof(ppcb_hit)), "pinned hits");
       check(cudaEventCreate(&S.t0), "event");
       check(cudaEventCreate(&S.t1), "event");
       S.busy = false;
@@ -184,6 +236,7 @@ void Engine::free_device(DeviceCtx& g) {
   cudaSetDevice(g.dev);
   g.back.reset();
   g.front.reset();
+  g.io.reset();
   if (g.st) cudaStreamSynchronize(g.st);
   if (g.cp) cudaStreamSynchronize(g.cp);
   void* ptrs[] = {g.absca, g.wmeta, g.lp, g.oms, g.az, g.sc, g.lr, g.ls, g.is, g.mcol, g.bfrt, g.sg_groups, g.sg_cells,
@@ -200,6 +253,7 @@ void Engine::free_device(DeviceCtx& g) {
     if (S.hb) cudaFreeHost(S.hb);
     if (S.hbstart) cudaFreeHost(S.hbstart);
     if (S.hctrl) cudaFreeHost(S.hctrl);
+    if (S.hfirst) cudaFreeHost(S.hfirst);
     if (S.t0) cudaEventDestroy(S.t0);
     if (S.t1) cudaEventDestroy(S.t1);
     S = DeviceCtx::Slot();
@@ -286,6 +340,9 @@ long Engine::submit(const ppcb_bunch* b, int nb, uint64_t num) {
       check(launch_propagate(a, g.shape, g.st), "propagate launch");
     }
     check(cudaMemcpyAsync(S.hctrl, S.ctrl, sizeof(ppcb_ctrl), cudaMemcpyDeviceToHost, g.st), "D2H ctrl");
+    if (acc > 0)
+      check(cudaMemcpyAsync(S.hfirst, S.hits, std::min<uint64_t>(kFirstHits, g.hcap) * sizeof(ppcb_hit),
+                            cudaMemcpyDeviceToHost, g.st), "D2H hits");
     check(cudaEventRecord(S.t1, g.st), "event");
     S.busy = true;
     g.next_slot ^= 1;
@@ -317,14 +374,16 @@ bool Engine::collect(const std::function<void(const ppcb_hit*, uint64_t)>& sink,
     const ppcb_ctrl c = *S->hctrl;
     uint64_t kept = std::min<uint64_t>(c.hidx, g.hcap);
     if (c.hidx > g.hcap) info.overflow = true;
-    if (kept > g.hhits_cap) {
-      cudaFreeHost(g.hhits);
-      g.hhits_cap = std::max<uint64_t>(kept, g.hhits_cap * 2);
-      check(cudaMallocHost((void**)&g.hhits, g.hhits_cap * sizeof(ppcb_hit)), "pinned hits");
-    }
-    if (kept) {
+    if (kept && kept <= kFirstHits) {
+      sink(S->hfirst, kept);
+    } else if (kept) {
+      if (kept > g.hhits_cap) {
+        cudaFreeHost(g.hhits);
+        g.hhits_cap = std::max<uint64_t>(kept, g.hhits_cap * 2);
+        check(cudaMallocHost((void**)&g.hhits, g.hhits_cap * sizeof(ppcb_hit)), "pinned hits");
+      }
       check(cudaMemcpyAsync(g.hhits, S->hits, kept * sizeof(ppcb_hit), cudaMemcpyDeviceToHost, g.cp), "D2H hits");
-      check(cudaStreamSynchronize(g.cp), "D2H hits");
+      g.io->wait(g.cp);
       sink(g.hhits, kept);
     }
     info.photons += S->num;

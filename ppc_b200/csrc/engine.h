@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <deque>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <functional>
 #include <vector>
@@ -28,8 +29,43 @@ struct RunInfo {
   bool overflow = false;
 };
 
+// Buffers of the host-pointer entry points (ppcb_accept, ppcb_sources, ppcb_llh_eval), kept
+// between calls: device memory in up to four parts and pinned staging memory.  Parts above
+// kKeepBytes, and staging above kStageBytes, are not kept: such a call's transfers take longer
+// than its allocations.  One call at a time uses them (`m`).
+class CallBuffers {
+ public:
+  static constexpr size_t kKeepBytes = 256u << 20, kStageBytes = 8u << 20;
+  std::mutex m;
+  void* device(int part, size_t bytes);  // at least `bytes`, on the current device
+  unsigned char* stage(size_t bytes);    // pinned; null above kStageBytes
+  // Waits for `st` on an event, as collect() does for a launch: a blocking stream wait wakes
+  // the caller some 200 us late.
+  void wait(cudaStream_t st);
+  ~CallBuffers();
+  // Held during a call: the lock, and at its end (or an error) what is not kept is given back.
+  struct Use {
+    explicit Use(CallBuffers& b) : lock(b.m), b_(b) {}
+    ~Use() { b_.trim(); }
+    std::lock_guard<std::mutex> lock;
+    CallBuffers& b_;
+  };
+
+ private:
+  void trim();
+  void* dev_[4] = {nullptr, nullptr, nullptr, nullptr};
+  size_t cap_[4] = {0, 0, 0, 0};
+  void* pin_ = nullptr;
+  size_t pin_cap_ = 0;
+  cudaEvent_t done_ = nullptr;
+};
+
 struct BackendTables;  // the device back end's sensor tables (backend.cu)
 struct FrontScratch;   // the device front end's per-source buffers (frontend.cu)
+
+// Hits that come back with a launch's control block, whether there are that many or not: a
+// call with fewer needs no second copy and wait (64 KB, 3 us).
+constexpr uint64_t kFirstHits = 2048;
 
 struct DeviceCtx {
   int dev = -1;
@@ -61,6 +97,7 @@ struct DeviceCtx {
     ppcb_hit* hits = nullptr;        // device
     ppcb_ctrl* ctrl = nullptr;       // device
     ppcb_ctrl* hctrl = nullptr;      // pinned
+    ppcb_hit* hfirst = nullptr;      // pinned: the first kFirstHits hits, copied with the control block
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     uint64_t num = 0;
     int nb = 0;
@@ -74,6 +111,7 @@ struct DeviceCtx {
   uint64_t hhits_cap = 0;
   std::shared_ptr<BackendTables> back;  // built on the first device back-end call
   std::shared_ptr<FrontScratch> front;  // grows to the largest device front-end call
+  std::shared_ptr<CallBuffers> io;      // the back end's and front end's host entry points
 };
 
 struct GradScratch;  // the gradient's device buffers (gradient.cu), kept between calls
@@ -138,7 +176,8 @@ class Engine {
   // one random stream per source; counts[0..1] (device) receive bunches needed and photons.
   void sources(int d, const ppcb_source* dsrc, uint64_t ns, uint32_t seed, ppcb_bunch* dout, uint64_t* dbstart,
                uint64_t cap, uint64_t* dcounts, cudaStream_t st);
-  int front_errors(int d);  // sources whose sampling failed, since ini (synchronises)
+  // Sources whose sampling failed, since ini: the device counter (null before the first call).
+  const int* front_errors(int d) const;
   // The back end's tables on device `d` (built from the configuration on first use).
   BackendTables& backend_tables(int d);
   double total_device_ms() const;
@@ -154,6 +193,12 @@ class Engine {
 };
 
 void check(cudaError_t e, const char* what);
+
+// Waits for what `st` has been given, of which `e` is recorded as the end: on the event for a
+// launch of up to kSpinPhotons photons (about 0.1 s), as collect() does, otherwise on the stream,
+// which leaves the core to others but wakes the caller some 200 us late.
+constexpr uint64_t kSpinPhotons = 100'000'000;
+void wait_launch(cudaStream_t st, cudaEvent_t e, uint64_t photons, const char* what);
 
 // One ice-fit iteration as a CUDA graph (gradient.cu): the recording forward pass, the charge
 // histogram, the Poisson weights and log-likelihood, and the replay of the detected photons

@@ -552,13 +552,9 @@ void Engine::sources(int d, const ppcb_source* dsrc, uint64_t ns, uint32_t seed,
   check(cudaGetLastError(), "front end write");
 }
 
-int Engine::front_errors(int d) {
-  DeviceCtx& g = devs.at(d);
-  if (!g.front) return 0;
-  check(cudaSetDevice(g.dev), "cudaSetDevice");
-  int e = 0;
-  check(cudaMemcpy(&e, g.front->errors, sizeof(int), cudaMemcpyDeviceToHost), "front end errors");
-  return e;
+const int* Engine::front_errors(int d) const {
+  const DeviceCtx& g = devs.at(d);
+  return g.front ? g.front->errors : nullptr;
 }
 
 }  // namespace ppcb

@@ -124,12 +124,14 @@ struct GradScratch {
   Pinned<unsigned int> hcounts, hstats;
   Pinned<double> hg, hll;
   Pinned<ppcb_ctrl> hctrl;
-  cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t e[3] = {nullptr, nullptr, nullptr}, end = nullptr;
   GradScratch() {
     for (auto& x : e) check(cudaEventCreate(&x), "event");
+    check(cudaEventCreateWithFlags(&end, cudaEventDisableTiming), "event");
   }
   ~GradScratch() {
     for (auto& x : e) if (x) cudaEventDestroy(x);
+    if (end) cudaEventDestroy(end);
   }
 };
 
@@ -223,7 +225,7 @@ Engine::Grad Engine::gradient(const ppcb_bunch* b, int nb, uint32_t events, cons
   check(cudaMemcpyAsync(X.hg.p, dgo.p, 2 * PPCB_MAXLYS * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H gradient");
   check(cudaMemcpyAsync(X.hstats.p, dstat.p, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st), "D2H stats");
   check(cudaMemcpyAsync(X.hctrl.p, dctrl.p, sizeof(ppcb_ctrl), cudaMemcpyDeviceToHost, st), "D2H ctrl");
-  check(cudaStreamSynchronize(st), "gradient");
+  wait_launch(st, X.end, bs[nb], "gradient");
   const ppcb_ctrl c = *X.hctrl.p;
   if (c.hidx > hit_cap) throw Error("gradient: hit capacity too small (" + std::to_string(c.hidx) + " hits)", 7);
   const uint64_t nh = c.hidx;
@@ -272,13 +274,14 @@ struct GradGraphState {
   Pinned<double> hg, hll;
   Pinned<unsigned int> hstats, hcounts;
   Pinned<ppcb_ctrl> hctrl;
-  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr}, end = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   ~GradGraphState() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     for (auto& x : ev) if (x) cudaEventDestroy(x);
+    if (end) cudaEventDestroy(end);
   }
 };
 
@@ -305,6 +308,7 @@ GradGraph::GradGraph(Engine& e, const ppcb_bunch* b, int nb, uint32_t events, co
   S.absca.need(e.cfg.absca.size());
   S.hg.need(2 * PPCB_MAXLYS); S.hll.need(1); S.hstats.need(2); S.hcounts.need(S.nbins); S.hctrl.need(1);
   for (auto& x : S.ev) check(cudaEventCreate(&x), "event");
+  check(cudaEventCreateWithFlags(&S.end, cudaEventDisableTiming), "event");
   cudaStream_t st = S.st;
   check(cudaMemcpyAsync(S.bunches.p, b, nb * sizeof(ppcb_bunch), cudaMemcpyHostToDevice, st), "H2D bunches");
   check(cudaMemcpyAsync(S.bstart.p, bs.data(), (nb + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st), "H2D");
@@ -372,7 +376,7 @@ Engine::Grad GradGraph::run(const float* be, const float* ba, bool counts) {
   e_.cfg.set_ice(be, ba);  // the table the graph uploads, then every other device's copy
   memcpy(S.absca.p, e_.cfg.absca.data(), e_.cfg.absca.size() * sizeof(float));
   check(cudaGraphLaunch(S.exec, S.st), "graph launch");
-  check(cudaStreamSynchronize(S.st), "gradient graph");
+  wait_launch(S.st, S.end, S.photons, "gradient graph");
   for (size_t k = 1; k < e_.devs.size(); k++) {
     check(cudaSetDevice(e_.devs[k].dev), "cudaSetDevice");
     check(cudaMemcpy(e_.devs[k].absca, S.absca.p, e_.cfg.absca.size() * sizeof(float), cudaMemcpyHostToDevice),

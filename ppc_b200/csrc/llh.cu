@@ -41,6 +41,7 @@ struct LlhDevice {
   int ndt_cap = 0;
   float2* list = nullptr;            // accepted hits (slot, time) of an evaluation in parts
   uint64_t list_cap = 0;
+  CallBuffers io;                    // host-pointer evaluations
   ~LlhDevice() {
     for (void* p : {(void*)dom_slot, (void*)doms, (void*)bin_block, (void*)block_dat, (void*)block_dom, (void*)win,
                     (void*)work, (void*)partial, (void*)errors, (void*)list})
@@ -467,6 +468,13 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   T.ndof = ndof;
   k_llh_terms<<<dim3(parts, ndt), kThreads, 0, st>>>(T);
   check(cudaGetLastError(), "likelihood terms");
+}
+
+CallBuffers& Likelihood::io() { return d_->io; }
+
+const int* Likelihood::device_errors() {
+  check(cudaSetDevice(eng_.devs.at(dev_).dev), "cudaSetDevice");
+  return d_->errors;
 }
 
 void Likelihood::require_device() {

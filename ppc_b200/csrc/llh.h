@@ -13,6 +13,7 @@
 namespace ppcb {
 
 class Engine;
+class CallBuffers;
 
 // One DOM that enters the likelihood (dat::in(), llh/llh.cxx:664-666), after dat::prep and
 // dat::optimize (llh/llh.cxx:436-450, 516-612).
@@ -47,6 +48,10 @@ class Likelihood {
   void eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, const double* dts, int ndt, double nsim,
                    double* dout, cudaStream_t st);
   int errors();  // llf evaluations that left their domain, since creation (synchronises)
+  // after require_device(): the error counter (its device made current) and the buffers of the
+  // host-pointer evaluation
+  const int* device_errors();
+  CallBuffers& io();
   void require_device();  // throws (status 6) before ppcb_ini(); uploads the tables
 
   ppcb_llh_opts opts;

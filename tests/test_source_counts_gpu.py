@@ -9,7 +9,7 @@ from conftest import have_gpu
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_gpu(), reason="needs a CUDA GPU")]
 
 from ppc_b200 import types as T  # noqa: E402
-from ppc_b200.api import PPC  # noqa: E402
+from ppc_b200.api import PPC, PPCError  # noqa: E402
 
 
 @pytest.fixture(scope="module")
@@ -135,3 +135,16 @@ def test_small_buffer_and_unaligned_output(ctx, cap):
         got = out.cpu().numpy()
         assert got[off:off + 64 * cap].tobytes() == whole[:cap].tobytes()
         assert not got[:off].any() and not got[off + 64 * cap:].any()
+
+
+@pytest.mark.parametrize("n", [3, 200_000])
+def test_failed_source_is_reported_once(ctx, n):
+    """A source that cannot be sampled fails its call (staged or not), not the next one."""
+    src = np.zeros(n, T.SOURCE_DTYPE)
+    src["kind"], src["amount"], src["q"] = T.SRC_POINT, 5, np.arange(n)
+    bad = src.copy()
+    bad["kind"][1], bad["type"][1] = T.SRC_PARTICLE, -1
+    with pytest.raises(PPCError):
+        ctx.sources(bad, seed=2)
+    bunches, _, photons = ctx.sources(src, seed=2)
+    assert len(bunches) == n and photons == 5 * n
