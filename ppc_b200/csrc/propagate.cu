@@ -1019,18 +1019,20 @@ struct PhotonPool {
 // sampled twice, costs 1/26 more.  Measured on the full detector's cascades without and with
 // it: 6e5 photons 1220 and 1104 us, 1e6 1634 and 1394, 3e6 3254 and 2776, 3e7 25810 and
 // 24970; 8 and 24 groups take 7% and 2% longer for 3e6, a kScreenU of 0.05 or 0.30 3% and 6%.
-// Below three photons per thread the launch lasts as long as its longest photon whenever
-// that starts (3e5 photons: 1045 us without, 1069 with it), and nothing is screened.
+// Below three photons per lane the launch lasts as long as its longest photon whenever that
+// starts, and nothing is screened.
 constexpr int kScreenGroups = 16;
 constexpr float kScreenU = 0.135f;
-constexpr uint64_t kScreenFrom = 3;  // photons per thread
+constexpr uint64_t kScreenFrom = 3;  // photons per lane
 
-// A launch of fewer photons than threads is dealt out over the SMs at its start, at best to
-// this many sixteenths of the warps (five per SM), a few lanes each: it is bound by the
-// latency of a step, 1.6 us for one lane, 2.2 us for a full warp and 3.6 us when every warp
-// of the SM is at work.  1000 photons 384 -> 283 us, 4096 630 -> 498, 3e4 785 -> 674 us
-// (with five sixteenths 4% more).
+// The warps at work.  The longest photon of a launch takes some 400 steps, of 1.6 us for a
+// lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them.  So a launch with
+// fewer photons than kLanePhotons for each lane uses fewer warps on every SM: its other photons
+// last as long as the longest one, and all steps are shorter.
+// And fewer photons than kFewWarps sixteenths of the warps (five per SM) have lanes are dealt
+// out over those warps at the start, a few lanes each.
 constexpr uint32_t kFewWarps = 3;
+constexpr uint64_t kLanePhotons = 6;
 
 // A warp's place in that order (shared memory; read and written by lane 0's turn only).
 struct WarpClaims {
@@ -1043,8 +1045,9 @@ struct WarpClaims {
 struct LaunchPlan {
   uint64_t num;  // photons
   int nb;        // bunches
-  int groups;    // screened groups per warp
-  int deal;      // fewer photons than threads: photons per warp, dealt at the start; else -1
+  uint32_t warps;  // warps at work, those of the lowest numbers
+  int groups;      // screened groups per warp
+  int deal;        // fewer photons than their lanes: photons per warp, dealt at the start; else -1
 };
 
 // Random streams.  Thread streams (STREAMS = false, the reference's scheme): each thread
@@ -1071,12 +1074,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   __shared__ LaunchPlan plan;
   if (threadIdx.x == 0) {
     bsteps = 0;
-    const uint32_t T = gridDim.x * BLOCK, few = max(1u, T / 32 * kFewWarps / 16);
     // launch sizes: from the parameters, or from device memory for replayed graphs
-    plan.num = a.dyn ? a.dyn[0] : a.num;
+    const uint64_t num = a.dyn ? a.dyn[0] : a.num;
+    const uint32_t warps = gridDim.x * (BLOCK / 32), few = max(1u, warps * kFewWarps / 16);
+    plan.num = num;
     plan.nb = a.dyn ? (int)a.dyn[1] : a.nb;
-    plan.groups = plan.num >= kScreenFrom * T ? (int)min((uint64_t)kScreenGroups, plan.num / T) : 0;
-    plan.deal = plan.num < T ? (int)min((uint64_t)32, (plan.num + few - 1) / few) : -1;
+    plan.warps = (uint32_t)max((uint64_t)few, min((uint64_t)warps, num / (32 * kLanePhotons)));
+    const uint64_t lanes = 32ull * plan.warps;
+    plan.groups = num >= kScreenFrom * lanes ? (int)min((uint64_t)kScreenGroups, num / lanes) : 0;
+    plan.deal = num < lanes ? (int)((num + plan.warps - 1) / plan.warps) : -1;
   }
   if (threadIdx.x < BLOCK / 32) {
     WarpClaims& c = s_claims[threadIdx.x];
@@ -1129,12 +1135,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
         uint64_t gidx = 0;
         float u = 0;
         // warps are numbered across the blocks first, so that few photons spread over all SMs
-        const uint32_t warps = T >> 5, gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        const uint32_t warps = plan.warps, gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
         if (fixed) {  // photon i on thread i mod T, as the oracle sequences it
           gen = !alive && s_sidx[threadIdx.x] < plan.num;
           gidx = s_sidx[threadIdx.x];
           if (!alive) s_sidx[threadIdx.x] += T;
           done = __all_sync(FULL, s_sidx[threadIdx.x] >= plan.num);
+        } else if (gw >= warps) {
+          done = true;
+          break;
         } else if (C.screened < plan.groups) {  // the next group to screen, once the pool is empty
           gen = screen = have == 0;
           gidx = ((uint64_t)C.screened * warps + gw) * 32 + lane;
@@ -1143,7 +1152,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
           unsigned long long base = (uint64_t)gw * n;
           if (plan.deal < 0) {
             if (lane == 0) base = atomicAdd(&a.ctrl->next, (unsigned long long)n);
-            base = (uint64_t)plan.groups * T + __shfl_sync(FULL, base, 0);
+            base = (uint64_t)plan.groups * warps * 32 + __shfl_sync(FULL, base, 0);
           }
           last = plan.deal >= 0 || base + n >= plan.num;
           gidx = base + lane;
