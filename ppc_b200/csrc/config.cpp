@@ -1061,8 +1061,8 @@ void Config::load(const std::string& tables_dir) {
 // String-proximity table (strgrid.h).  Lines on the same axis form a group (its disc covers
 // theirs, widened by kReachPad); a square grid over the groups' footprint plus a
 // 64 m margin, with cells as small as kSgMaxCells allows (from 8 m up), stores per cell the
-// nearest group and a lower bound on the distance from the cell to every other group's
-// widened disc (exact on the cell square, rounded down to kSgClearUnit).  Not part of the
+// nearest group and a lower bound on the squared distance from the cell to every other group's
+// widened disc (exact on the cell square, rounded down to the entry's float).  Not part of the
 // reference's tables: it only decides when the reference's DOM search can be skipped.
 void Config::build_strgrid() {
   sg = StrGridParams{};
@@ -1100,18 +1100,23 @@ void Config::build_strgrid() {
     cell *= 1.25;
   }
   const double ox = x0 - margin, oy = y0 - margin;
-  sg.inv = (float)(1 / cell);
-  sg.ou = (float)(-ox / cell);
-  sg.ov = (float)(-oy / cell);
-  sg.margin2 = (float)(margin * margin);
+  nx = std::max(nx, 2);
+  ny = std::max(ny, 2);
+  sg.su = (float)(1 / ((nx - 1) * cell));
+  sg.sv = (float)(1 / ((ny - 1) * cell));
+  sg.ou = (float)(-(ox + cell / 2) / ((nx - 1) * cell));
+  sg.ov = (float)(-(oy + cell / 2) / ((ny - 1) * cell));
+  sg.cu = nx - 1;
+  sg.cv = ny - 1;
   sg.nx = nx; sg.ny = ny; sg.on = 1;
+  sg.base = (int32_t)(0u - (uint32_t)kSgMagicBits * (uint32_t)(nx + 1));
   sg_cells.assign((size_t)nx * ny, 0);
   for (int j = 0; j < ny; j++)
     for (int i = 0; i < nx; i++) {
-      // the cell of the device's index arithmetic, widened by a millimetre on each side
+      // the cell of the device's index arithmetic, widened by two millimetres on each side
       // (the index is computed in single precision from the origin and the cell size)
-      const double xa = ox + i * cell - 1e-3, xb = ox + (i + 1) * cell + 1e-3;
-      const double ya = oy + j * cell - 1e-3, yb = oy + (j + 1) * cell + 1e-3;
+      const double xa = ox + i * cell - 2e-3, xb = ox + (i + 1) * cell + 2e-3;
+      const double ya = oy + j * cell - 2e-3, yb = oy + (j + 1) * cell + 2e-3;
       int best = -1;
       double d1 = 1e30, d2 = 1e30;  // nearest and second-nearest disc distance
       for (int k = 0; k < ng; k++) {
@@ -1121,9 +1126,11 @@ void Config::build_strgrid() {
         if (d < d1) { d2 = d1; d1 = d; best = k; }
         else if (d < d2) d2 = d;
       }
-      const double q = std::floor(d2 / kSgClearUnit);
-      const unsigned int clear = q > 255 ? 255u : (unsigned int)q;
-      sg_cells[(size_t)j * nx + i] = (uint16_t)((clear << 8) | (unsigned int)(best < 0 ? ng : best));
+      // the largest code whose float, with every bit below it set, is at most the square of
+      // the clearance; code 0 stands for less than 0.4 cm, which kReachPad covers
+      uint32_t code = 255;
+      while (code > 0 && sg_float(((code + 1) << 20) + kSgClearBase) > d2 * d2) code--;
+      sg_cells[(size_t)j * nx + i] = (uint16_t)((code << 8) | (unsigned int)(best < 0 ? ng : best));
     }
   sg_groups.push_back(StrGroup{1e30f, 1e30f, 0, 0});  // the sentinel: no group within reach
 }
