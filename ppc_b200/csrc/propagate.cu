@@ -727,7 +727,9 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
   int J;
   float nr = 1.f;
   {
-    if (TOT > 0) {  // absorption anisotropy, gpu/pro.cu:517-544
+    // absorption anisotropy, gpu/pro.cu:517-544 (without a branch for the photons vetoed at
+    // emission, TOT = 0, which take no path at all)
+    {
       float2 n12 = __ffma2_rn(make_float2(e.azx, -e.azy), make_float2(n.x, n.x),
                               __fmul2_rn(make_float2(e.azy, e.azx), make_float2(n.y, n.y)));
       float n1 = n12.x, n2 = n12.y;
@@ -746,7 +748,7 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
       n12 = __fmul2_rn(n12, make_float2(e.k1, e.k2));
       n1 = n12.x; n2 = n12.y; n3 *= e.kz;
       nr *= rsqrtf(n1 * n1 + n2 * n2 + n3 * n3);
-      TOT /= nr;
+      TOT = TOT > 0 ? TOT / nr : TOT;
     }
     float ahx = edh * (0.5f - sign * (z - I));
     J = I;  // layer stepping, gpu/pro.cu:548-571
@@ -754,10 +756,11 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
     float2 ts = make_float2(0.f, 0.f);   // (tot, sca)
     float2 aa = make_float2(TOT, SCA);   // (aia, ais)
     float2 c = ice(wz, J);
+    const int Jend = sign < 0 ? 0 : e.size - 1;
     while (true) {
       float dsca = aa.y / c.y, dtot = aa.x / c.x;
       float dist = fminf(dsca, dtot) * anz;
-      if ((sign < 0 ? J > 0 : J < e.size - 1) && dist > ahx) {
+      if (J != Jend && dist > ahx) {
         float del = ahx / anz;
         ts = __fadd2_rn(ts, make_float2(del, del));
         aa = __ffma2_rn(c, make_float2(-del, -del), aa);
@@ -822,19 +825,22 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
   else {
     if (e.sum > 0 && fin > 0) {  // birefringence diffusion, gpu/pro.cu:757-836
       float ra, rb;
-      if (I == J) {
-        const float2 q = __fmul2_rn(make_float2(fin, fin), make_float2(S.az[I].ra, S.az[I].rb));
-        ra = q.x; rb = q.y;
-      }
-      else {
+      // one layer, or the parts of two and (rarely) the layers between, both formed by every
+      // lane and then selected: a warp has lanes of either kind (+1.3%)
+      {
+        const ppcb_aniz aI = S.az[I], aJ = S.az[J];
+        const float2 q = __fmul2_rn(make_float2(fin, fin), make_float2(aI.ra, aI.rb));
         float y = z + n.z * fin / edh;
         float h = 0.5f - sign * (z - I);
         float g = 0.5f + sign * (y - J);
-        ra = h * S.az[I].ra + g * S.az[J].ra;
-        rb = h * S.az[I].rb + g * S.az[J].rb;
-        for (int i = I + sign; i != J && (unsigned)i < (unsigned)e.size; i += sign) { ra += S.az[i].ra; rb += S.az[i].rb; }
+        ra = h * aI.ra + g * aJ.ra;
+        rb = h * aI.rb + g * aJ.rb;
+        if ((unsigned)(I - J + 1) > 2u)
+          for (int i = I + sign; i != J && (unsigned)i < (unsigned)e.size; i += sign) { ra += S.az[i].ra; rb += S.az[i].rb; }
         float f = edh / anz;
         ra *= f; rb *= f;
+        ra = I == J ? q.x : ra;
+        rb = I == J ? q.y : rb;
       }
       if (ra < 0) ra = 0;
       if (rb < 0) rb = 0;
@@ -905,16 +911,17 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
       SCA = 0;
       const float4 c0 = S.scat[hole][0], c1 = S.scat[hole][1];
       float xi = xrnd(s);
-      if (xi > c0.x) {
-        xi = (1 - xi) * c0.w;
-        xi = 2 * xi - 1;
-        if (c0.y != 0) {
-          float ga = c1.x / (1 + c0.y * xi);
-          xi = (ga * ga - c1.y) * c1.z;
-        }
-      } else {
-        xi *= c1.w;
-        xi = 2 * (1 - powf(xi, c0.z));
+      // the Henyey-Greenstein and the SAM mapping, both for every lane: a warp has lanes of
+      // either kind and would run them one after the other around a branch (+1.8%)
+      {
+        float xh = (1 - xi) * c0.w;
+        xh = 2 * xh - 1;
+        const float ga = c1.x / (1 + c0.y * xh);
+        const float xg = (ga * ga - c1.y) * c1.z;
+        xh = c0.y != 0 ? xg : xh;
+        float xs = xi * c1.w;
+        xs = 2 * (1 - powf(xs, c0.z));
+        xi = xi > c0.x ? xh : xs;
       }
       if (xi < 0) xi = 0;
       else if (xi > 2) xi = 2;
@@ -1027,10 +1034,11 @@ constexpr uint64_t kScreenFrom = 3;  // photons per lane
 
 // The warps at work.  The longest photon of a launch takes some 400 steps, of 1.6 us for a
 // lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them.  So a launch with
-// fewer photons than kLanePhotons for each lane uses fewer warps on every SM: its other photons
-// last as long as the longest one, and all steps are shorter.
-// And fewer photons than kFewWarps sixteenths of the warps (five per SM) have lanes are dealt
-// out over those warps at the start, a few lanes each.
+// fewer photons than kLanePhotons for each lane uses fewer warps on every SM, whose steps are
+// shorter: 1e5 photons 872 -> 844 us, 3e5 1038 -> 947, 6e5 1100 -> 1050, 1e6 (all warps) 1393;
+// with 13 per lane 3e5 take 1155 and 1e6 1426 us.  Fewer photons than kFewWarps sixteenths of
+// the warps (five per SM) have lanes are dealt out over those warps at the start, a few lanes
+// each: 1000 photons 384 -> 283 us, 4096 630 -> 498, 3e4 785 -> 674 (five sixteenths: +4%).
 constexpr uint32_t kFewWarps = 3;
 constexpr uint64_t kLanePhotons = 6;
 
@@ -1111,6 +1119,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   // index in the static order and the last bunch found
   __shared__ uint64_t s_sidx[BLOCK];
   __shared__ int s_hint[BLOCK];
+  __shared__ uint32_t s_steps[BLOCK];  // steps of the thread's finished photons
+  s_steps[threadIdx.x] = 0;
   s_sidx[threadIdx.x] = gt;
   s_hint[threadIdx.x] = 0;
   unsigned int nan_steps = 0;
@@ -1261,17 +1271,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
     if (alive) {
       step(a, S, dt, ph, s, nan_steps, hk);
       ph.steps++;
-      if (a.max_steps && ph.steps >= a.max_steps && ph.TOT != 0) {  // the step cap (rare)
+      if (ph.steps > a.max_steps - 1u && ph.TOT != 0) {  // the step cap (rare; 0: none)
         ph.TOT = 0;
         atomicAdd(&a.ctrl->capped, 1u);
       }
-      if (ph.TOT == 0) {  // the photon's steps go to the block's count
+      if (ph.TOT == 0) {  // (a 64-bit atomic of the block's count is a loop: 1.3% of the kernel)
         alive = false;
-        atomicAdd(&bsteps, (unsigned long long)ph.steps);
+        s_steps[threadIdx.x] += ph.steps;
       }
     }
   }
   if constexpr (!STREAMS) a.rs[gt] = (uint64_t)s.x | ((uint64_t)s.y << 32);
+  atomicAdd(&bsteps, (unsigned long long)s_steps[threadIdx.x]);
   __syncthreads();
   if (threadIdx.x == 0) atomicAdd(&a.ctrl->steps, bsteps);
 }

@@ -1,6 +1,6 @@
-"""The order in which a launch takes its photons: dealt out at the start (fewer photons than
-threads), from the queue, or screened by absorption depth first (three photons per thread and
-more).  Whatever the order, every photon is propagated exactly once, with its own random
+"""The order in which a launch takes its photons: dealt out at the start (few photons), from
+the queue, or screened by absorption depth first (three photons per lane and more), on some
+or all of the warps.  Whatever the order, every photon is propagated exactly once, with its own random
 numbers."""
 import numpy as np
 import pytest
@@ -30,14 +30,14 @@ def _iso(num, q=1):
 
 def _sizes(threads):
     return [1, 31, 32, 33, 749, 750, 751, 23_968, 23_969, threads - 1, threads, threads + 1, 3 * threads - 1, 3 * threads,
-            3 * threads + 1, 17 * threads + 5]
+            3 * threads + 1, 17 * threads + 5, 144_000, 6 * threads - 1, 6 * threads + 1]
 
 
 def _sorted(h):
     return np.sort(np.ascontiguousarray(h).view("V32").ravel())
 
 
-@pytest.mark.parametrize("k", range(16))
+@pytest.mark.parametrize("k", range(19))
 def test_every_photon_once(ice_small, k):
     """The hits of a launch of n photons are the hits of the first n photons of a larger launch
     (another order: photon i draws from its own stream wherever it runs)."""
