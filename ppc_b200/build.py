@@ -13,6 +13,7 @@ bit for bit (see tests/test_config_pin.py).
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
@@ -34,6 +35,9 @@ CXXFLAGS = ["-O2", "-ffp-contract=off", "-fPIC", "-std=c++17", "-Wall", "-Wno-un
 
 CU = ["propagate.cu", "engine.cu", "noalloc.cu", "batch.cu", "gradient.cu", "peak.cu", "backend.cu", "llh.cu",
       "frontend.cu"]
+# propagate.cu again for each tilt model's kernels (its TiltKind): an object each, so that they
+# compile side by side
+PARTS = [("propagate.cu", k) for k in range(4)]
 CPP = ["config.cpp", "session.cpp", "capi.cpp", "capi_batch.cpp", "capi_llh.cpp", "xppc.cpp", "llh.cpp"]
 # Fast math everywhere but in the front end, whose bunch templates follow the host front
 # end's float arithmetic (no approximate logf/powf, no contraction).  The likelihood
@@ -69,14 +73,17 @@ def build(verbose=False):
     os.makedirs(LIB, exist_ok=True)
     os.makedirs(BIN, exist_ok=True)
     hdrs = [os.path.join(SRC, h) for h in HEADERS] + [os.path.join(INC, "ppc_b200.h"), os.path.join(INC, "xppc.h")]
-    objs = []
-    for f in CU:
-        src, obj = os.path.join(SRC, f), os.path.join(OBJ, f + ".o")
+    objs, cmds = [], []
+    for f, k in [(f, None) for f in CU] + PARTS:
+        name = f if k is None else f"{f}.{k}"
+        src, obj = os.path.join(SRC, f), os.path.join(OBJ, name + ".o")
         if _newer(obj, [src] + hdrs):
-            fast = [] if f in CU_EXACT else CU_FAST_MATH
-            _run([NVCC] + NVFLAGS + fast + CU_EXTRA.get(f, []) + ["-c", src, "-o", obj],
-                 log=os.path.join(OBJ, f + ".ptxas.txt"))
+            flags = ([] if f in CU_EXACT else CU_FAST_MATH) + CU_EXTRA.get(f, [])
+            flags += [] if k is None else [f"-DPPCB_TILT={k}"]
+            cmds.append(([NVCC] + NVFLAGS + flags + ["-c", src, "-o", obj], os.path.join(OBJ, name + ".ptxas.txt")))
         objs.append(obj)
+    with ThreadPoolExecutor(max(1, min(8, os.cpu_count() or 1))) as pool:
+        list(pool.map(lambda c: _run(*c), reversed(cmds)))  # the longest first
     for f in CPP:
         src, obj = os.path.join(SRC, f), os.path.join(OBJ, f + ".o")
         if _newer(obj, [src] + hdrs):
@@ -100,8 +107,9 @@ def build(verbose=False):
     if _newer(mwc, [mwc_src]):
         _run(["gcc", "-O2", "-fopenmp", mwc_src, "-o", mwc])
     if verbose:
-        with open(os.path.join(OBJ, "propagate.cu.ptxas.txt")) as f:
-            sys.stdout.write(f.read())
+        for _, k in PARTS:
+            with open(os.path.join(OBJ, f"propagate.cu.{k}.ptxas.txt")) as f:
+                sys.stdout.write(f.read())
     return os.path.join(LIB, "libppcb.so")
 
 

@@ -1,7 +1,9 @@
 // Device runtime (see engine.h).
 #include "engine.h"
+#include "tilt.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -188,6 +190,10 @@ void Engine::ini() {
     upload(g.mcol, cfg.mcol.data(), PPCB_CTX * PPCB_CTY, "mcol");
     g.bfrt = dalloc<float4>(PPCB_BFR_TAB + 1, "bfrt");
     upload(g.bfrt, (const float4*)cfg.bfrt.data(), PPCB_BFR_TAB + 1, "bfrt");
+    std::vector<float2> cells;
+    tilt_tables(cells);
+    g.tcell = dalloc<float2>(kTiltCells, "tilt cells");
+    upload(g.tcell, cells.data(), kTiltCells, "tilt cells");
     if (cfg.sg.on) {
       g.sg_groups = dalloc<StrGroup>(cfg.sg_groups.size(), "sg_groups");
       upload(g.sg_groups, cfg.sg_groups.data(), cfg.sg_groups.size(), "sg_groups");
@@ -239,11 +245,11 @@ void Engine::free_device(DeviceCtx& g) {
   g.io.reset();
   if (g.st) cudaStreamSynchronize(g.st);
   if (g.cp) cudaStreamSynchronize(g.cp);
-  void* ptrs[] = {g.absca, g.wmeta, g.lp, g.oms, g.az, g.sc, g.lr, g.ls, g.is, g.mcol, g.bfrt, g.sg_groups, g.sg_cells,
+  void* ptrs[] = {g.absca, g.wmeta, g.lp, g.oms, g.az, g.sc, g.lr, g.ls, g.is, g.mcol, g.bfrt, g.sg_groups, g.sg_cells, g.tcell,
                   g.rs, g.rm};
   for (void* p : ptrs) if (p) cudaFree(p);
   g.absca = nullptr; g.wmeta = nullptr; g.lp = nullptr; g.oms = nullptr; g.az = nullptr; g.sc = nullptr;
-  g.bfrt = nullptr; g.sg_groups = nullptr; g.sg_cells = nullptr;
+  g.bfrt = nullptr; g.tcell = nullptr; g.sg_groups = nullptr; g.sg_cells = nullptr;
   g.lr = nullptr; g.ls = nullptr; g.is = nullptr; g.mcol = nullptr; g.rs = nullptr; g.rm = nullptr;
   for (auto& S : g.slot) {
     if (S.bunches) cudaFree(S.bunches);
@@ -275,6 +281,40 @@ void Engine::fin() {
   inited_ = false;
 }
 
+// The 1-d cells over the inner radii lr[1..lnum-2] and a metre on either side: per cell the
+// only radius that may lie in it (infinity: none) and the number of the interval below it.
+// A cell is widened by a hundredth of itself for the rounding of a point's cell number.
+void Engine::tilt_tables(std::vector<float2>& cells) {
+  const ppcb_params& p = cfg.p;
+  tilt_ = TiltFast{0.f, 0.f, {0.f, 0.f}, 0};
+  cells.assign(kTiltCells, make_float2(INFINITY, 0.f));
+  if (p.tmod == 2) {
+    tilt_.on = tilt_recip_ok(p.mstp[0]) && tilt_recip_ok(p.mstp[1]);
+    for (int i = 0; i < 2; i++) tilt_.rstep[i] = 1 / p.mstp[i];
+  }
+  if (p.tmod != 1 || p.lnum < 2) return;
+  const auto& lr = cfg.lr;
+  for (int k = 1; k < p.lnum; k++)
+    if (!tilt_recip_ok(lr[k] - lr[k - 1])) return;
+  const double lo = p.lnum > 2 ? lr[1] - 1.0 : lr[0], hi = p.lnum > 2 ? lr[p.lnum - 2] + 1.0 : lr[1];
+  const double w = (hi - lo) / (kTiltCells - 1);
+  tilt_.scale = (float)(1 / (hi - lo));
+  tilt_.off = (float)(-lo / (hi - lo));
+  for (int c = 0; c < kTiltCells; c++) {
+    int below = 0, inside = 0;
+    for (int k = 1; k < p.lnum - 1; k++) {
+      if (c > 0 && lr[k] < lo + (c - 0.51) * w) below++;
+      else if (c == kTiltCells - 1 || lr[k] <= lo + (c + 0.51) * w) inside++;
+    }
+    if (inside > 1) return;
+    const int j = 1 + below;
+    float jf;
+    memcpy(&jf, &j, sizeof(jf));
+    cells[c] = make_float2(inside ? lr[j] : INFINITY, jf);
+  }
+  tilt_.on = 1;
+}
+
 KArgs Engine::args_for(int d) const {
   const DeviceCtx& g = devs[d];
   KArgs a;
@@ -284,6 +324,8 @@ KArgs Engine::args_for(int d) const {
   a.lr = g.lr; a.ls = g.ls; a.is = g.is; a.mcol = g.mcol; a.bfrt = g.bfrt;
   a.sg = cfg.sg; a.sg_groups = g.sg_groups; a.sg_ngroups = (int)cfg.sg_groups.size(); a.sg_cells = g.sg_cells;
   if (!a.sg_cells) a.sg.on = 0;
+  a.tf = tilt_;
+  a.tcell = g.tcell;
   a.rs = g.rs; a.rm = g.rm;
   a.deterministic = deterministic;
   a.seed = sv;

@@ -85,6 +85,7 @@ struct DeviceCtx {
   uint16_t* is = nullptr;
   int8_t* mcol = nullptr;
   float4* bfrt = nullptr;
+  float2* tcell = nullptr;         // 1-d tilt interval cells (tilt.h)
   StrGroup* sg_groups = nullptr;   // string-proximity table (strgrid.h)
   uint16_t* sg_cells = nullptr;
   uint64_t* rs = nullptr;
@@ -185,6 +186,8 @@ class Engine {
 
  private:
   void free_device(DeviceCtx& g);
+  void tilt_tables(std::vector<float2>& cells);
+  TiltFast tilt_{};
   std::shared_ptr<GradScratch> gs_;  // grows to the largest gradient call; freed by fin()
   bool inited_ = false;
   bool initialized_ = false;

@@ -333,7 +333,7 @@ GradGraph::GradGraph(Engine& e, const ppcb_bunch* b, int nb, uint32_t events, co
   KArgs r = e.args_for(0);
   r.ctrl = S.ctrl.p;
   const unsigned long long* nh_dev = &S.ctrl.p->hidx;
-  check(adjoint_prepare(), "replay attribute");
+  check(adjoint_prepare(r), "replay attribute");
 
   // the timing events are recorded as external event nodes, so that a replay records them
   check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");

@@ -23,7 +23,14 @@ namespace {
 
 struct HostTilt {
   const Config& c;
-  float lr(int i) const { return c.lr[i]; }
+  int interval(float nr) const { return tilt_interval(c.p.lnum, [this](int i) { return c.lr[i]; }, nr); }
+  float4 span(int j) const {
+    float4 v;
+    v.x = c.lr[j - 1]; v.y = c.lr[j]; v.z = c.lr[j] - c.lr[j - 1]; v.w = 0;
+    return v;
+  }
+  static constexpr bool kRecip = false, kConstantLayers = false;
+  float rstep(int) const { return 0; }
   int mcol(int x, int y) const {
     return x >= 0 && x < c.p.mnum[0] && y >= 0 && y < c.p.mnum[1] ? c.mcol[x * PPCB_CTY + y] : -1;
   }

@@ -40,12 +40,13 @@ namespace ppcb {
 #define OMR PPCB_OMR
 #define WNUM PPCB_WNUM
 
-__device__ __constant__ float kFcv = PPCB_FPI / 180.f;
+static __device__ __constant__ float kFcv = PPCB_FPI / 180.f;
 
 struct SmemTables {
   ppcb_aniz az[PPCB_MAXLYS];
   ppcb_line sc[PPCB_NSTR];
-  float lr[PPCB_LMAX];
+  float4 span[PPCB_LMAX];         // 1-d tilt map interval j: lr[j-1], lr[j], difference, reciprocal
+  float2 tcell[kTiltCells];       // 1-d tilt: where to find the interval (TiltFast)
   uint16_t ls[PPCB_NSTR];
   uint16_t is[PPCB_CX * PPCB_CY];
   int8_t mcol[PPCB_CTX * PPCB_CTY];
@@ -88,7 +89,7 @@ __device__ __forceinline__ void photon_stream(Rng& s, uint64_t i, uint32_t seed)
 }
 
 // gpu/pro.cu:59-85
-__device__ float mrnd(float k, Rng& s) {
+static __device__ float mrnd(float k, Rng& s) {
   float x;
   if (k < 1) {
     float c = 1 / k;
@@ -187,23 +188,54 @@ __device__ __forceinline__ void normalize3(float4& n) {
 }
 
 // ---------------------------------------------------------------- index helpers
-// tilt tables as seen by the kernel: radii and map columns in shared memory, the
+// The kernels are compiled for each ice model: code of another model in the step's loop, even
+// if it is never run, costs instruction fetches (with both tilt models, their divisions and the
+// interval search behind uniform branches 1e3 photons take 258 us and 3e7 22470, with one of
+// them 230 and 21710; hole ice and the anisotropy's power law behind branches another 2%).
+// A model is a TiltKind, plus kPlain for ice without hole ice and without that power law.
+enum TiltKind {
+  kNoTilt,
+  kTilt1D, kTilt2D,  // with TiltFast's quotients and cells, layers of constant thickness
+  kTiltAny           // any model as the reference computes it
+};
+constexpr int kPlain = 4;
+__host__ __device__ constexpr int tilt_of(int model) { return model & 3; }
+__host__ __device__ constexpr bool plain(int model) { return model & kPlain; }
+
+// tilt tables as seen by the kernel: map intervals and map columns in shared memory, the
 // depth maps through the read-only cache
+template <bool FAST>
 struct DevTilt {
   const SmemTables& S;
+  const KArgs& a;
   const ppcb_params& d;
   const float2* __restrict__ lpg;
-  __device__ __forceinline__ float lr(int i) const { return S.lr[i]; }
+  __device__ __forceinline__ int interval(float nr) const {
+    if constexpr (FAST) {
+      const float u = __saturatef(fmaf(nr, a.tf.scale, a.tf.off));
+      const float2 c = S.tcell[__float_as_int(fmaf(u, kTiltCells - 1.f, kSgMagic)) - kSgMagicBits];
+      return __float_as_int(c.y) + !(nr < c.x);
+    } else {
+      return tilt_interval(d.lnum, [this](int i) { return i ? S.span[i].y : S.span[1].x; }, nr);
+    }
+  }
+  __device__ __forceinline__ float4 span(int j) const { return S.span[j]; }
+  __device__ __forceinline__ float rstep(int i) const { return a.tf.rstep[i]; }
+  static constexpr bool kRecip = FAST, kConstantLayers = FAST;
   __device__ __forceinline__ int mcol(int x, int y) const {
     return x >= 0 && x < d.mnum[0] && y >= 0 && y < d.mnum[1] ? S.mcol[x * PPCB_CTY + y] : -1;
   }
   __device__ __forceinline__ float2 lp(int i, int k) const { return __ldg(&lpg[i * PPCB_LYRS + k]); }
 };
 
-__device__ __forceinline__ float zshift(const ppcb_params& d, const SmemTables& S, const float2* __restrict__ lp,
-                                        float rx, float ry, float rz, float& dz) {
-  DevTilt t{S, d, lp};
-  return zshift_t(d, t, rx, ry, rz, dz);
+template <int MODEL>
+__device__ __forceinline__ float zshift(const KArgs& a, const SmemTables& S, float rx, float ry, float rz, float& dz) {
+  constexpr int TILT = tilt_of(MODEL);
+  const DevTilt<TILT != kTiltAny> t{S, a, a.p, a.lp};
+  if constexpr (TILT == kTilt1D) return zshift_1d_t(a.p, t, rx, ry, rz, dz);
+  else if constexpr (TILT == kTilt2D) return zshift_2d_t(a.p, t, rx, ry, rz, dz);
+  else if constexpr (TILT == kTiltAny) return zshift_t(a.p, t, rx, ry, rz, dz);
+  else return 0;
 }
 
 // gpu/pro.cu:507-515: tilt-corrected depth in layer units and the current layer.
@@ -391,7 +423,7 @@ struct Sampled {
   uint32_t x, y;  // stream state after the draws
 };
 
-__device__ __noinline__ Sampled sample_photon(const KArgs& a, int bunch, uint32_t sx, uint32_t sy, uint32_t sa) {
+static __device__ __noinline__ Sampled sample_photon(const KArgs& a, int bunch, uint32_t sx, uint32_t sy, uint32_t sa) {
   Rng s;
   s.x = sx; s.y = sy; s.a = sa;
   Sampled out;
@@ -402,7 +434,7 @@ __device__ __noinline__ Sampled sample_photon(const KArgs& a, int bunch, uint32_
 }
 
 // gpu/pro.cu:734-745: the hit record (photon and DOM-surface angles)
-__device__ __noinline__ ppcb_hit hit_record(const KArgs& a, int om, float4 r, float4 n, float sqd, uint32_t niw,
+static __device__ __noinline__ ppcb_hit hit_record(const KArgs& a, int om, float4 r, float4 n, float sqd, uint32_t niw,
                                            int wl) {
   const ppcb_params& e = a.p;
   ppcb_hit h;
@@ -446,7 +478,7 @@ __device__ __forceinline__ unsigned long long emit_hit(const KArgs& a, const ppc
 }
 
 // the plain kernel's hit append, out of line (about one step in 2e4 registers a hit)
-__device__ __noinline__ void emit_hit_cold(const KArgs& a, ppcb_hit h) { emit_hit(a, h); }
+static __device__ __noinline__ void emit_hit_cold(const KArgs& a, ppcb_hit h) { emit_hit(a, h); }
 
 // ---------------------------------------------------------------- step hooks
 // The plain propagation: hits are appended, nothing else is observed.
@@ -535,7 +567,7 @@ struct AdjHook {
 // gpu/pro.cu:655-669: entry and exit of the segment in the hole-ice column of a string
 // (radius hr), given the string's closest-approach terms b, c and np = 1 - nz^2; returns
 // the updated (hi, hf).
-__device__ __noinline__ float2 hole_column(const ppcb_params& e, float b, float c, float np, float sca, float hi,
+static __device__ __noinline__ float2 hole_column(const ppcb_params& e, float b, float c, float np, float sca, float hi,
                                            float hf) {
   float DH = b * b - (c - e.hr2) * np;
   if (DH > 0) {
@@ -560,7 +592,7 @@ struct Truncated {
 
 // gpu/pro.cu:677-717: a step cut short at fin (DOM hit or hole-ice entry): the optical
 // depths used over the bulk-ice part by layers, then the hole-ice part.
-__device__ __noinline__ Truncated truncated_step(const ppcb_params& e, const float2* __restrict__ wz, float z, float nz,
+static __device__ __noinline__ Truncated truncated_step(const ppcb_params& e, const float2* __restrict__ wz, float z, float nz,
                                                  float fin, float edh, int I, int sign, float anz, float SCA,
                                                  float TOT, float nr, float hi, float hf, float del, float sca,
                                                  int om) {
@@ -602,7 +634,7 @@ __device__ __noinline__ Truncated truncated_step(const ppcb_params& e, const flo
 
 // gpu/pro.cu:728: a step with a non-finite optical depth is counted (and the first four SMs
 // where it happened recorded); the photon is then dropped by the caller
-__device__ __noinline__ void record_nan_step(const KArgs& a) {
+static __device__ __noinline__ void record_nan_step(const KArgs& a) {
   unsigned int k = atomicAdd(&a.ctrl->nan_steps, 1u);
   if (k < 4) { unsigned int sm; asm volatile("mov.u32 %0, %%smid;" : "=r"(sm)); a.ctrl->bad_sm[k] = sm; }
 }
@@ -636,6 +668,7 @@ struct Found {
 // order (cells, then the strings of each cell, then the DOM window of each string).  It
 // runs only for the steps the string-proximity table cannot rule out.  Inlined: as a call
 // it would make the step save and restore its live registers around the call site.
+template <int MODEL>
 __device__ __forceinline__ Found dom_search(const KArgs& a, const SmemTables& S, float4 r, float4 n, float sca, int old,
                                          int ofla) {
   const ppcb_params& e = a.p;
@@ -644,7 +677,7 @@ __device__ __forceinline__ Found dom_search(const KArgs& a, const SmemTables& S,
   {  // DOM search, gpu/pro.cu:577-672
     int xlx, xhx, xly, xhy;
     cell_range(e, r.x, r.y, fa(r.x, fm(sca, n.x)), fa(r.y, fm(sca, n.y)), xlx, xhx, xly, xhy);
-    const bool hole_on = e.hr > 0 && (e.hifl == 0 || (e.hifl < 0 && r.w < -e.hifl) || (e.hifl > 0 && r.w > e.hifl));
+    const bool hole_on = !plain(MODEL) && e.hr > 0 && (e.hifl == 0 || (e.hifl < 0 && r.w < -e.hifl) || (e.hifl > 0 && r.w > e.hifl));
     for (int i = xlx, j = xly; i <= xhx && j <= xhy; (++j <= xhy) ? 0 : (j = xly, i++)) {
       for (unsigned int k = S.is[i * PPCB_CY + j]; k != 0x8000;) {
         unsigned int m = S.ls[k];
@@ -706,7 +739,7 @@ __device__ __forceinline__ Found dom_search(const KArgs& a, const SmemTables& S,
 
 // gpu/pro.cu:499-888: one propagation step (one scattering segment).  Returns with
 // ph.TOT == 0 once the photon is absorbed or registered.
-template <class HOOK>
+template <int MODEL, class HOOK>
 __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const DynTabs& dt, Photon& ph, Rng& s,
                                      unsigned int& nan_steps, HOOK& hk) {
   const ppcb_params& e = a.p;
@@ -721,7 +754,7 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
   int sign = n.z < 0 ? -1 : 1;
   float anz = sign * n.z;
   float edh = e.dh;
-  float zs = zshift(e, S, a.lp, r.x, r.y, r.z, edh);
+  float zs = zshift<MODEL>(a, S, r.x, r.y, r.z, edh);
   float z;
   int I = layer_of(e, r.z, zs, z);
   int J;
@@ -734,7 +767,7 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
                               __fmul2_rn(make_float2(e.azy, e.azx), make_float2(n.y, n.y)));
       float n1 = n12.x, n2 = n12.y;
       float n3 = n.z;
-      if (e.fr != 0) {
+      if (!plain(MODEL) && e.fr != 0) {
         float k1 = S.az[I].k1, k2 = S.az[I].k2;
         float kz = 1 / (k1 * k2);
         float s1 = n1 * n1, l1 = k1 * k1;
@@ -785,9 +818,10 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
   // DOM search, gpu/pro.cu:577-672: only for the steps that may reach a string's cylinder
   // (strgrid.h; on the full detector about 0.2% of them); for the others it would find
   // nothing and leave om, del, hi, hf and sqd as they are
-  if (sg_may_reach(a.sg, SgTab{S, dt.cells}, r.x, r.y, n.x, n.y, n.z, sca)) {
-    const Found f = dom_search(a, S, r, n, sca, old, ph.ofla);
-    om = f.om; del = f.del; hi = f.hi; hf = f.hf; sqd = f.sqd;
+  if (__builtin_expect(sg_may_reach(a.sg, SgTab{S, dt.cells}, r.x, r.y, n.x, n.y, n.z, sca), 0)) {
+    const Found f = dom_search<MODEL>(a, S, r, n, sca, old, ph.ofla);
+    om = f.om; del = f.del; sqd = f.sqd;
+    if constexpr (!plain(MODEL)) { hi = f.hi; hf = f.hf; }
   }
 
   float fin = fminf(del, hi);
@@ -875,7 +909,7 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
       const float pz = n.x * qxy.y - n.y * qxy.x;
       float2 rnd = grnd2(s);
       float2 dn = __ffma2_rn(sxy, rnd, make_float2(mx, 0.f));
-      if (del <= hi) {  // curved path within the segment
+      if (plain(MODEL) || del <= hi) {  // curved path within the segment
         rnd = grnd2(s);
         float2 vn = __fmul2_rn(__ffma2_rn(__fmul2_rn(sxy, rnd), make_float2(rsqrtf(3.f), rsqrtf(3.f)), dn),
                                make_float2(0.5f, 0.5f));
@@ -953,7 +987,11 @@ __device__ __forceinline__ void load_tables(const KArgs& a, SmemTables& S) {
   const int nt = blockDim.x, t = threadIdx.x;
   for (int i = t; i < a.p.size; i += nt) S.az[i] = a.az[i];
   for (int i = t; i < a.p.nstr; i += nt) S.sc[i] = a.sc[i];
-  for (int i = t; i < PPCB_LMAX; i += nt) S.lr[i] = a.lr[i];
+  for (int i = t; i < kTiltCells; i += nt) S.tcell[i] = a.tcell[i];
+  for (int i = t + 1; i < PPCB_LMAX; i += nt) {
+    const float lo = a.lr[i - 1], hi = a.lr[i], w = __fsub_rn(hi, lo);
+    S.span[i] = make_float4(lo, hi, w, __fdiv_rn(1.f, w));
+  }
   for (int i = t; i < PPCB_NSTR; i += nt) S.ls[i] = a.ls[i];
   for (int i = t; i < PPCB_CX * PPCB_CY; i += nt) S.is[i] = a.is[i];
   for (int i = t; i < PPCB_CTX * PPCB_CTY; i += nt) S.mcol[i] = a.mcol[i];
@@ -1071,7 +1109,7 @@ __host__ __device__ constexpr size_t dyn_smem() {
   return (BLOCK / 32) * sizeof(PhotonPool<STREAMS>) + (REC ? BLOCK * sizeof(Prov) : 0);
 }
 
-template <int BLOCK, int MINB, bool REC, bool STREAMS>
+template <int BLOCK, int MINB, bool REC, bool STREAMS, int MODEL>
 __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant__ KArgs a) {
   __shared__ SmemTables S;
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1269,7 +1307,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
     }
     if (!__any_sync(FULL, alive)) break;
     if (alive) {
-      step(a, S, dt, ph, s, nan_steps, hk);
+      step<MODEL>(a, S, dt, ph, s, nan_steps, hk);
       ph.steps++;
       if (ph.steps > a.max_steps - 1u && ph.TOT != 0) {  // the step cap (rare; 0: none)
         ph.TOT = 0;
@@ -1300,6 +1338,7 @@ __device__ __forceinline__ long long charge_bin(const ppcb_hit& h, uint32_t even
 // the path's per-layer derivative terms, weighted by the hit's DOM weight, until the
 // recorded hit is reached again.  A replay that does not end on the recorded hit (same
 // DOM, same time bits) is counted in stats[1].
+template <int MODEL>
 __global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_constant__ KArgs a, const ppcb_hit* __restrict__ hits,
                                                  const Prov* __restrict__ prov, uint64_t cap,
                                                  const unsigned long long* nh_dev, uint32_t events,
@@ -1349,7 +1388,7 @@ __global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_con
     hk.prov_out = nullptr;
     hk.start = nullptr;
     while (!hk.done && ph.TOT != 0 && ph.steps < a.max_steps) {
-      step(a, S, dt, ph, s, nan_steps, hk);
+      step<MODEL>(a, S, dt, ph, s, nan_steps, hk);
       ph.steps++;
     }
     replayed++;
@@ -1364,6 +1403,74 @@ __global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_con
   if (unmatched) atomicAdd(&stats[1], unmatched);
 }
 
+// Sets a kernel's dynamic shared-memory limit, once per device (a function attribute; it has to
+// be set before any stream capture that launches the kernel there).
+template <class K>
+static cudaError_t allow_smem(std::atomic<uint64_t>& done, K kernel, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(done.load() & bit)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    done.fetch_or(bit);
+  }
+  return cudaSuccess;
+}
+
+// The launches of a model's kernels.  Each tilt kind's kernels are an object file of their own
+// (this file compiled with PPCB_TILT set to the kind); the object without it dispatches.
+template <int MODEL>
+cudaError_t model_adjoint_prepare();
+template <int MODEL>
+cudaError_t model_adjoint(const KArgs& a, const ppcb_hit* hits, const void* prov, uint64_t nh, uint32_t events,
+                          const float* wdom, const float2* wgrad, double* g_out, unsigned int* stats, int blocks,
+                          cudaStream_t st, const unsigned long long* nh_dev);
+template <int MODEL>
+cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st);
+template <int MODEL>
+cudaError_t model_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f, cudaStream_t st);
+template <int MODEL>
+int model_max_blocks(int threads);
+template <int MODEL>
+int model_rec_blocks(int threads, bool streams);
+
+#ifndef PPCB_TILT
+// The model of a launch.
+static int model_of(const KArgs& a) {
+  int t = a.p.tmod == 1 ? kTilt1D : a.p.tmod == 2 ? kTilt2D : kNoTilt;
+  if (t != kNoTilt && (!a.tf.on || a.p.vthk != 0)) return kTiltAny;
+  return t | (!(a.p.hr > 0) && a.p.fr == 0 ? kPlain : 0);
+}
+
+// Calls f with the launch's model as a compile-time constant.
+template <class F>
+static auto with_model(const KArgs& a, F&& f) {
+  switch (model_of(a)) {
+    case kNoTilt: return f(std::integral_constant<int, kNoTilt>());
+    case kTilt1D: return f(std::integral_constant<int, kTilt1D>());
+    case kTilt2D: return f(std::integral_constant<int, kTilt2D>());
+    case kNoTilt | kPlain: return f(std::integral_constant<int, kNoTilt | kPlain>());
+    case kTilt1D | kPlain: return f(std::integral_constant<int, kTilt1D | kPlain>());
+    case kTilt2D | kPlain: return f(std::integral_constant<int, kTilt2D | kPlain>());
+    default: return f(std::integral_constant<int, kTiltAny>());
+  }
+}
+
+cudaError_t adjoint_prepare(const KArgs& a) {
+  return with_model(a, [](auto m) { return model_adjoint_prepare<decltype(m)::value>(); });
+}
+
+cudaError_t launch_adjoint(const KArgs& a, const ppcb_hit* hits, const void* prov, uint64_t nh, uint32_t events,
+                           const float* wdom, const float2* wgrad, double* g_out, unsigned int* stats, int blocks,
+                           cudaStream_t st, const unsigned long long* nh_dev) {
+  if (nh == 0) return cudaSuccess;
+  return with_model(a, [&](auto m) {
+    return model_adjoint<decltype(m)::value>(a, hits, prov, nh, events, wdom, wgrad, g_out, stats, blocks, st, nh_dev);
+  });
+}
+
 __global__ void k_dom_hist(const ppcb_hit* __restrict__ hits, uint64_t cap, const unsigned long long* nh_dev,
                            unsigned int* counts, uint32_t events, int gsize) {
   const uint64_t nh = nh_dev ? (*nh_dev < cap ? *nh_dev : cap) : cap;
@@ -1373,39 +1480,16 @@ __global__ void k_dom_hist(const ppcb_hit* __restrict__ hits, uint64_t cap, cons
   }
 }
 
-// The replay's static shared memory plus the string-proximity table exceed the default
-// 48 KiB of dynamic shared memory: allow the largest table, once per device (before any
-// stream capture that launches the replay there).
-cudaError_t adjoint_prepare() {
-  static std::atomic<uint64_t> done{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (!(done.load() & (1ull << (dev & 63)))) {
-    e = cudaFuncSetAttribute(k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(kSgMaxCells * sizeof(uint16_t) + kBfrBytes));
-    if (e != cudaSuccess) return e;
-    done.fetch_or(1ull << (dev & 63));
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_adjoint(const KArgs& a, const ppcb_hit* hits, const void* prov, uint64_t nh, uint32_t events,
-                           const float* wdom, const float2* wgrad, double* g_out, unsigned int* stats, int blocks,
-                           cudaStream_t st, const unsigned long long* nh_dev) {
-  if (nh == 0) return cudaSuccess;
-  const cudaError_t e = adjoint_prepare();
-  if (e != cudaSuccess) return e;
-  k_adjoint<<<blocks, 256, sg_cells_bytes(a) + kBfrBytes, st>>>(a, hits, static_cast<const Prov*>(prov), nh, nh_dev, events,
-                                                   wdom, wgrad, g_out, stats);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_dom_hist(const ppcb_hit* hits, uint64_t nh, unsigned int* counts, uint32_t events, int gsize,
                             cudaStream_t st, const unsigned long long* nh_dev) {
   if (nh == 0) return cudaSuccess;
   k_dom_hist<<<592, 256, 0, st>>>(hits, nh, nh_dev, counts, events, gsize);
   return cudaGetLastError();
+}
+
+cudaError_t launch_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st) {
+  if (a.deterministic < 0 || a.deterministic > 2) return cudaErrorInvalidValue;
+  return with_model(a, [&](auto m) { return model_propagate<decltype(m)::value>(a, sh, st); });
 }
 
 // Phase-1 only: thread t samples photon t with stream t (test entry point).
@@ -1427,9 +1511,33 @@ __global__ void __launch_bounds__(PPCB_BLOCK) k_generate(const __grid_constant__
   a.rs[gt] = (uint64_t)s.x | ((uint64_t)s.y << 32);
 }
 
+cudaError_t launch_generate(const KArgs& a, LaunchShape, void* pbuf_out, cudaStream_t st) {
+  int blocks = (int)((a.num + PPCB_BLOCK - 1) / PPCB_BLOCK);
+  if (blocks == 0) return cudaSuccess;
+  k_generate<<<blocks, PPCB_BLOCK, 0, st>>>(a, (float4*)pbuf_out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f,
+                               cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  return with_model(a, [&](auto m) { return model_index_probe<decltype(m)::value>(a, pos, n, out_i, out_f, st); });
+}
+
+// The models' kernels have the same launch bounds and shared memory: the general one stands for
+// them all.
+int propagate_rec_blocks_per_sm(int threads, int deterministic) {
+  return model_rec_blocks<kTiltAny>(threads, deterministic != 1);
+}
+
+int propagate_max_blocks_per_sm(int threads) { return model_max_blocks<kTiltAny>(threads); }
+
+#else   // PPCB_TILT
+
 // Index helpers at given points (test entry point).  pos[2k] = (x,y,z,t) start,
 // pos[2k+1] = (nx,ny,nz,len) direction and segment length.  Outputs per point:
 // ints  [layer, xlx, xhx, xly, xhy, n1, n2, string]   floats [zshift, dz]
+template <int MODEL>
 __global__ void k_index_probe(const __grid_constant__ KArgs a, const float4* pos, int np, int32_t* oi, float* of) {
   __shared__ SmemTables S;
   load_tables(a, S);
@@ -1437,7 +1545,7 @@ __global__ void k_index_probe(const __grid_constant__ KArgs a, const float4* pos
   if (k >= np) return;
   const float4 r = pos[2 * k], n = pos[2 * k + 1];
   float dz = a.p.dh;
-  float zs = zshift(a.p, S, a.lp, r.x, r.y, r.z, dz);
+  float zs = zshift<MODEL>(a, S, r.x, r.y, r.z, dz);
   float z;
   int I = layer_of(a.p, r.z, zs, z);
   int xlx, xhx, xly, xhy;
@@ -1460,74 +1568,129 @@ __global__ void k_index_probe(const __grid_constant__ KArgs a, const float4* pos
 // that memory to the L1 cache.  Per-photon streams run with
 // deterministic = 2, and in the gradient's recording pass unless the photon order is
 // static (deterministic = 1: thread streams, photon i on thread i mod T, nothing interleaves).
-// The dynamic shared-memory limit is a per-device function attribute: set it once on each
-// device (before any stream capture that launches the kernel there).
 // Dynamic shared memory: the photon pools (and provenance slots), then the
 // string-proximity cell entries; the attribute allows the largest table.
-template <int BLOCK, int MINB, bool REC, bool STREAMS>
+template <int BLOCK, int MINB, bool REC, bool STREAMS, int MODEL>
 static cudaError_t launch_one(const KArgs& a, int blocks, cudaStream_t st) {
   constexpr size_t dmax = dyn_smem<BLOCK, REC, STREAMS>() + kSgMaxCells * sizeof(uint16_t) + kBfrBytes;
   const size_t dyn = dyn_smem<BLOCK, REC, STREAMS>() + sg_cells_bytes(a) + kBfrBytes;
   if (dyn > dmax) return cudaErrorInvalidValue;
   static std::atomic<uint64_t> done{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const cudaError_t e = allow_smem(done, k_propagate<BLOCK, MINB, REC, STREAMS, MODEL>, dmax);
   if (e != cudaSuccess) return e;
-  const uint64_t bit = 1ull << (dev & 63);
-  if (!(done.load() & bit)) {
-    e = cudaFuncSetAttribute(k_propagate<BLOCK, MINB, REC, STREAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)dmax);
-    if (e != cudaSuccess) return e;
-    done.fetch_or(bit);
-  }
-  k_propagate<BLOCK, MINB, REC, STREAMS><<<blocks, BLOCK, dyn, st>>>(a);
+  k_propagate<BLOCK, MINB, REC, STREAMS, MODEL><<<blocks, BLOCK, dyn, st>>>(a);
   return cudaGetLastError();
 }
 
-template <bool REC, bool STREAMS>
+template <bool REC, bool STREAMS, int MODEL>
 static cudaError_t launch_shape(const KArgs& a, LaunchShape sh, cudaStream_t st) {
   if constexpr (REC) {
     switch (sh.threads) {
-      case 256: return launch_one<256, 3, true, STREAMS>(a, sh.blocks, st);
-      case 864: return launch_one<864, 1, true, STREAMS>(a, sh.blocks, st);
+      case 256: return launch_one<256, 3, true, STREAMS, MODEL>(a, sh.blocks, st);
+      case 864: return launch_one<864, 1, true, STREAMS, MODEL>(a, sh.blocks, st);
       default: return cudaErrorInvalidConfiguration;
     }
   } else {
     switch (sh.threads) {
-      case 256: return launch_one<256, 3, false, STREAMS>(a, sh.blocks, st);
-      case 128: return launch_one<128, 6, false, STREAMS>(a, sh.blocks, st);
-      case 768: return launch_one<768, 1, false, STREAMS>(a, sh.blocks, st);
-      case 864: return launch_one<864, 1, false, STREAMS>(a, sh.blocks, st);
+      case 256: return launch_one<256, 3, false, STREAMS, MODEL>(a, sh.blocks, st);
+      case 128: return launch_one<128, 6, false, STREAMS, MODEL>(a, sh.blocks, st);
+      case 768: return launch_one<768, 1, false, STREAMS, MODEL>(a, sh.blocks, st);
+      case 864: return launch_one<864, 1, false, STREAMS, MODEL>(a, sh.blocks, st);
       default: return cudaErrorInvalidConfiguration;
     }
   }
 }
 
-cudaError_t launch_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st) {
-  if (a.deterministic < 0 || a.deterministic > 2) return cudaErrorInvalidValue;
+template <int MODEL>
+cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st) {
   if (a.prov) {
-    return a.deterministic == 1 ? launch_shape<true, false>(a, sh, st) : launch_shape<true, true>(a, sh, st);
+    return a.deterministic == 1 ? launch_shape<true, false, MODEL>(a, sh, st)
+                                : launch_shape<true, true, MODEL>(a, sh, st);
   }
-  return a.deterministic == 2 ? launch_shape<false, true>(a, sh, st) : launch_shape<false, false>(a, sh, st);
+  return a.deterministic == 2 ? launch_shape<false, true, MODEL>(a, sh, st)
+                              : launch_shape<false, false, MODEL>(a, sh, st);
 }
 
-cudaError_t launch_generate(const KArgs& a, LaunchShape, void* pbuf_out, cudaStream_t st) {
-  int blocks = (int)((a.num + PPCB_BLOCK - 1) / PPCB_BLOCK);
-  if (blocks == 0) return cudaSuccess;
-  k_generate<<<blocks, PPCB_BLOCK, 0, st>>>(a, (float4*)pbuf_out);
+// The replay's static shared memory plus the string-proximity table exceed the default
+// 48 KiB of dynamic shared memory: allow the largest table.
+template <int MODEL>
+cudaError_t model_adjoint_prepare() {
+  static std::atomic<uint64_t> done{0};
+  return allow_smem(done, k_adjoint<MODEL>, kSgMaxCells * sizeof(uint16_t) + kBfrBytes);
+}
+
+template <int MODEL>
+cudaError_t model_adjoint(const KArgs& a, const ppcb_hit* hits, const void* prov, uint64_t nh, uint32_t events,
+                          const float* wdom, const float2* wgrad, double* g_out, unsigned int* stats, int blocks,
+                          cudaStream_t st, const unsigned long long* nh_dev) {
+  const cudaError_t e = model_adjoint_prepare<MODEL>();
+  if (e != cudaSuccess) return e;
+  k_adjoint<MODEL><<<blocks, 256, sg_cells_bytes(a) + kBfrBytes, st>>>(a, hits, static_cast<const Prov*>(prov), nh,
+                                                                       nh_dev, events, wdom, wgrad, g_out, stats);
   return cudaGetLastError();
 }
 
-cudaError_t launch_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f,
-                               cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  k_index_probe<<<(n + 255) / 256, 256, 0, st>>>(a, pos, n, out_i, out_f);
+template <int MODEL>
+cudaError_t model_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f,
+                              cudaStream_t st) {
+  k_index_probe<MODEL><<<(n + 255) / 256, 256, 0, st>>>(a, pos, n, out_i, out_f);
   return cudaGetLastError();
 }
+
+// Resident blocks per SM of a kernel with `dyn` bytes of dynamic shared memory; 0 when it does
+// not fit.
+template <class K>
+static int resident_blocks(K kernel, int threads, size_t dyn) {
+  int nb = 0;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, dyn);
+  if (e != cudaSuccess) { cudaGetLastError(); return 0; }
+  return nb;
+}
+
+template <int BLOCK, int MINB, bool REC, bool STREAMS, int MODEL>
+static int shape_blocks() {  // with the larger pool (per-photon streams) and the largest string-proximity table
+  return resident_blocks(k_propagate<BLOCK, MINB, REC, STREAMS, MODEL>, BLOCK,
+                         dyn_smem<BLOCK, REC, STREAMS || !REC>() + kSgMaxCells * sizeof(uint16_t) + kBfrBytes);
+}
+
+template <int MODEL>
+int model_max_blocks(int threads) {
+  switch (threads) {
+    case 128: return shape_blocks<128, 6, false, false, MODEL>();
+    case 256: return shape_blocks<256, 3, false, false, MODEL>();
+    case 768: return shape_blocks<768, 1, false, false, MODEL>();
+    case 864: return shape_blocks<864, 1, false, false, MODEL>();
+    default: return 0;
+  }
+}
+
+template <int MODEL>
+int model_rec_blocks(int threads, bool streams) {
+  switch (threads) {
+    case 256: return streams ? shape_blocks<256, 3, true, true, MODEL>() : shape_blocks<256, 3, true, false, MODEL>();
+    case 864: return streams ? shape_blocks<864, 1, true, true, MODEL>() : shape_blocks<864, 1, true, false, MODEL>();
+    default: return 0;
+  }
+}
+
+#define PPCB_MODEL_LAUNCHES(M)                                                                                       \
+  template cudaError_t model_adjoint_prepare<M>();                                                                   \
+  template cudaError_t model_adjoint<M>(const KArgs&, const ppcb_hit*, const void*, uint64_t, uint32_t, const float*, \
+                                        const float2*, double*, unsigned int*, int, cudaStream_t,                    \
+                                        const unsigned long long*);                                                  \
+  template cudaError_t model_propagate<M>(const KArgs&, LaunchShape, cudaStream_t);                                  \
+  template cudaError_t model_index_probe<M>(const KArgs&, const float4*, int, int32_t*, float*, cudaStream_t);
+PPCB_MODEL_LAUNCHES(PPCB_TILT)
+#if PPCB_TILT < 3
+PPCB_MODEL_LAUNCHES(PPCB_TILT | kPlain)
+#else
+template int model_max_blocks<PPCB_TILT>(int);
+template int model_rec_blocks<PPCB_TILT>(int, bool);
 
 cudaError_t propagate_attributes(int* regs, int* max_threads, size_t* smem, size_t* local) {
   cudaFuncAttributes at;
-  cudaError_t e = cudaFuncGetAttributes(&at, k_propagate<256, 3, false, false>);
+  cudaError_t e = cudaFuncGetAttributes(&at, k_propagate<256, 3, false, false, kTiltAny>);
   if (e != cudaSuccess) return e;
   *regs = at.numRegs;
   *max_threads = at.maxThreadsPerBlock;
@@ -1535,49 +1698,8 @@ cudaError_t propagate_attributes(int* regs, int* max_threads, size_t* smem, size
   *local = at.localSizeBytes;
   return cudaSuccess;
 }
+#endif
 
-template <int BLOCK, int MINB>
-static int max_blocks(int* nb) {
-  // the larger pool (per-photon streams) and the largest string-proximity table
-  constexpr size_t dyn = dyn_smem<BLOCK, false, true>() + kSgMaxCells * sizeof(uint16_t) + kBfrBytes;
-  cudaError_t e = cudaFuncSetAttribute(k_propagate<BLOCK, MINB, false, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_propagate<BLOCK, MINB, false, false>, BLOCK, dyn);
-  return e == cudaSuccess ? *nb : 0;
-}
-
-// Resident blocks per SM of the gradient's recording kernel (its provenance slots and the
-// largest string-proximity table included); 0 when the shape does not fit.
-template <int BLOCK, int MINB, bool STREAMS>
-static int rec_blocks(int* nb) {
-  constexpr size_t dyn = dyn_smem<BLOCK, true, STREAMS>() + kSgMaxCells * sizeof(uint16_t) + kBfrBytes;
-  cudaError_t e = cudaFuncSetAttribute(k_propagate<BLOCK, MINB, true, STREAMS>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_propagate<BLOCK, MINB, true, STREAMS>, BLOCK, dyn);
-  if (e != cudaSuccess) { cudaGetLastError(); return 0; }
-  return *nb;
-}
-
-int propagate_rec_blocks_per_sm(int threads, int deterministic) {
-  int nb = 0;
-  const bool streams = deterministic != 1;
-  switch (threads) {
-    case 256: return streams ? rec_blocks<256, 3, true>(&nb) : rec_blocks<256, 3, false>(&nb);
-    case 864: return streams ? rec_blocks<864, 1, true>(&nb) : rec_blocks<864, 1, false>(&nb);
-    default: return 0;
-  }
-}
-
-int propagate_max_blocks_per_sm(int threads) {
-  int nb = 0;
-  switch (threads) {
-    case 128: return max_blocks<128, 6>(&nb);
-    case 256: return max_blocks<256, 3>(&nb);
-    case 768: return max_blocks<768, 1>(&nb);
-    case 864: return max_blocks<864, 1>(&nb);
-    default: return 0;
-  }
-}
+#endif  // PPCB_TILT
 
 }  // namespace ppcb

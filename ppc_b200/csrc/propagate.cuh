@@ -5,6 +5,7 @@
 
 #include "ppcb_types.h"
 #include "strgrid.h"
+#include "tilt.h"
 
 namespace ppcb {
 
@@ -18,7 +19,7 @@ struct KArgs {
   const ppcb_dom* oms;       // [gsize]
   const ppcb_aniz* az;       // [size]        -> shared memory
   const ppcb_line* sc;       // [nstr]        -> shared memory
-  const float* lr;           // [LMAX]        -> shared memory
+  const float* lr;           // [LMAX]        -> shared memory, as the intervals' spans
   const uint16_t* ls;        // [NSTR]        -> shared memory
   const uint16_t* is;        // [CX*CY]       -> shared memory
   const int8_t* mcol;        // [CTX*CTY]     -> shared memory
@@ -26,6 +27,8 @@ struct KArgs {
   StrGridParams sg;          // string-proximity table (strgrid.h); sg.on = 0: no strings
   const StrGroup* sg_groups; // [sg_ngroups]  -> shared memory
   int sg_ngroups;
+  TiltFast tf;               // tilt: what replaces the divisions and the interval search
+  const float2* tcell;       // [kTiltCells] -> shared memory (1-d)
   const uint16_t* sg_cells;  // [nx*ny]       -> shared memory (dynamic)
   // work
   const ppcb_bunch* bunches; // [nb]
@@ -75,7 +78,8 @@ cudaError_t launch_adjoint(const KArgs& a, const ppcb_hit* hits, const void* pro
 cudaError_t launch_dom_hist(const ppcb_hit* hits, uint64_t nh, unsigned int* counts, uint32_t events, int gsize,
                             cudaStream_t st, const unsigned long long* nh_dev = nullptr);
 constexpr int kAdjointPerSm = 3;  // resident blocks of the replay per SM
-cudaError_t adjoint_prepare();  // the replay's launch attribute on the current device (before a capture)
+// the replay's launch attribute on the current device (before a capture)
+cudaError_t adjoint_prepare(const KArgs& a);
 constexpr size_t kProvBytes = 64;  // provenance record per hit slot of the gradient's recording pass
 cudaError_t propagate_attributes(int* regs, int* max_threads, size_t* smem, size_t* local);
 int propagate_max_blocks_per_sm(int threads);
