@@ -144,38 +144,52 @@ __device__ __forceinline__ float2 grnd2(Rng& s) {
 
 __device__ __forceinline__ void swp(float& a, float& b) { float t = a; a = b; b = t; }
 
-// gpu/pro.cu:111-153: rotate n by polar angle (cs = 1-cos, si = sin), uniform azimuth
+__device__ __forceinline__ float sum_sq(float x, float y, float z) {
+  return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
+}
+
+// gpu/pro.cu:111-153: rotate n by polar angle (cs = 1-cos, si = sin), uniform azimuth.
+// The largest component comes first by selects: the lanes of a warp have it in all three
+// places, and around branches they would run one after the other (3e7 photons 21.2 -> 20.6 ms,
+// 1e3 213 -> 205 us).  The sums are fused in a fixed way, the one that the compiler chose for
+// the branches: with any other the photons' paths change in the last bits.
 __device__ __forceinline__ void rotate(float cs, float si, float4& n, Rng& s) {
   float3 p1, p2;
-  int i = 0;
+  float q1x;
+  int i;
   {
     float3 r;
     r.x = n.x * n.x; r.y = n.y * n.y; r.z = n.z * n.z;
-    if (r.y > r.z) {
-      if (r.y > r.x) { swp(n.x, n.y); swp(r.x, r.y); i = 1; }
-    } else {
-      if (r.z > r.x) { swp(n.x, n.z); swp(r.x, r.z); i = 2; }
-    }
-    r.y = rsqrtf(r.x + r.y); p1.x = -n.y * r.y; p1.y = n.x * r.y; p1.z = 0;
-    r.z = rsqrtf(r.x + r.z); p2.x = -n.z * r.z; p2.y = 0; p2.z = n.x * r.z;
+    const bool yz = r.y > r.z, xy = yz & (r.y > r.x), xz = !yz & (r.z > r.x);
+    const float nx = xy ? n.y : xz ? n.z : n.x, rx = xy ? r.y : xz ? r.z : r.x;
+    n.y = xy ? n.x : n.y; r.y = xy ? r.x : r.y;
+    n.z = xz ? n.x : n.z; r.z = xz ? r.x : r.z;
+    n.x = nx;
+    i = xy ? 1 : xz ? 2 : 0;
+    r.y = rsqrtf(__fadd_rn(rx, r.y)); p1.y = n.x * r.y; p1.z = 0;
+    r.z = rsqrtf(__fadd_rn(rx, r.z)); p2.x = __fmul_rn(-n.z, r.z); p2.y = 0; p2.z = n.x * r.z;
+    q1x = __fmaf_rn(-n.y, r.y, -p2.x); p2.x = __fmaf_rn(-n.y, r.y, p2.x);  // p1.x = -n.y r.y
   }
   {
     float3 q1;
-    q1.x = p1.x - p2.x; q1.y = p1.y - p2.y; q1.z = p1.z - p2.z;
-    p2.x += p1.x; p2.y += p1.y; p2.z += p1.z;
-    float w = rsqrtf(q1.x * q1.x + q1.y * q1.y + q1.z * q1.z);
+    q1.x = q1x; q1.y = p1.y - p2.y; q1.z = p1.z - p2.z;
+    p2.y += p1.y; p2.z += p1.z;
+    float w = rsqrtf(sum_sq(q1.x, q1.y, q1.z));
     p1.x = q1.x * w; p1.y = q1.y * w; p1.z = q1.z * w;
-    w = rsqrtf(p2.x * p2.x + p2.y * p2.y + p2.z * p2.z);
+    w = rsqrtf(sum_sq(p2.x, p2.y, p2.z));
     p2.x *= w; p2.y *= w; p2.z *= w;
   }
   {
     float2 p;
     float xi = xrnd_angle(s);
     sincosf(xi, &p.y, &p.x);
-    n.x -= cs * n.x - si * (p.x * p1.x + p.y * p2.x);
-    n.y -= cs * n.y - si * (p.x * p1.y + p.y * p2.y);
-    n.z -= cs * n.z - si * (p.x * p1.z + p.y * p2.z);
-    float r = rsqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
+    const auto turned = [&](float v, float a, float b) {
+      return __fsub_rn(v, __fmaf_rn(cs, v, -__fmul_rn(si, __fmaf_rn(p.y, b, __fmul_rn(p.x, a)))));
+    };
+    n.x = turned(n.x, p1.x, p2.x);
+    n.y = turned(n.y, p1.y, p2.y);
+    n.z = turned(n.z, p1.z, p2.z);
+    float r = rsqrtf(sum_sq(n.y, n.x, n.z));
     n.x *= r; n.y *= r; n.z *= r;
     if (i == 1) swp(n.x, n.y);
     else if (i == 2) swp(n.x, n.z);
@@ -1074,11 +1088,14 @@ constexpr uint64_t kScreenFrom = 3;  // photons per lane
 // lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them.  So a launch with
 // fewer photons than kLanePhotons for each lane uses fewer warps on every SM, whose steps are
 // shorter: 1e5 photons 872 -> 844 us, 3e5 1038 -> 947, 6e5 1100 -> 1050, 1e6 (all warps) 1393;
-// with 13 per lane 3e5 take 1155 and 1e6 1426 us.  Fewer photons than kFewWarps sixteenths of
+// with 13 per lane 3e5 take 1155 and 1e6 1426 us.  In hole ice the step is longer and depends
+// less on the warps beside it, so there kLanePhotonsHole holds (a point source in the column
+// with 2 and with 6 per lane: 1.2e5 photons 687 and 864 us, 4e5 958 and 1064; without hole ice
+// 4e5 836 and 764).  Fewer photons than kFewWarps sixteenths of
 // the warps (five per SM) have lanes are dealt out over those warps at the start, a few lanes
 // each: 1000 photons 384 -> 283 us, 4096 630 -> 498, 3e4 785 -> 674 (five sixteenths: +4%).
 constexpr uint32_t kFewWarps = 3;
-constexpr uint64_t kLanePhotons = 6;
+constexpr uint64_t kLanePhotons = 6, kLanePhotonsHole = 2;
 
 // A warp's place in that order (shared memory; read and written by lane 0's turn only).
 struct WarpClaims {
@@ -1125,7 +1142,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
     const uint32_t warps = gridDim.x * (BLOCK / 32), few = max(1u, warps * kFewWarps / 16);
     plan.num = num;
     plan.nb = a.dyn ? (int)a.dyn[1] : a.nb;
-    plan.warps = (uint32_t)max((uint64_t)few, min((uint64_t)warps, num / (32 * kLanePhotons)));
+    plan.warps = (uint32_t)max((uint64_t)few, min((uint64_t)warps, num / (32 * (!plain(MODEL) && a.p.hr > 0 ? kLanePhotonsHole : kLanePhotons))));
     const uint64_t lanes = 32ull * plan.warps;
     plan.groups = num >= kScreenFrom * lanes ? (int)min((uint64_t)kScreenGroups, num / lanes) : 0;
     plan.deal = num < lanes ? (int)((num + plan.warps - 1) / plan.warps) : -1;

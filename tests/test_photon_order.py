@@ -52,6 +52,20 @@ def test_every_photon_once(ice_small, k):
     c.close()
 
 
+@pytest.mark.parametrize("k", range(6))
+def test_every_photon_once_in_hole_ice(ice_small_hole, k):
+    """The same where hole ice has more warps at work for a given number of photons."""
+    c = _ctx(ice_small_hole, photon_streams=True)
+    threads = c.info()["threads"]
+    n = [47_935, 47_937, 120_000, 2 * threads - 1, 2 * threads + 1, 6 * threads + 1][k]
+    small, info = c.propagate(_iso(n))
+    large, _ = c.propagate(np.concatenate([_iso(n), _iso(7 * threads + 77, q=2)]))
+    part = large[large["n"] == 1]
+    assert info["photons"] == n and len(small) == len(part) > 0
+    assert np.array_equal(_sorted(small), _sorted(part))
+    c.close()
+
+
 @pytest.mark.parametrize("mult", [0.5, 2, 3, 17.3])
 def test_thread_streams_keep_the_absorption_law(ice_small, mult):
     """Thread streams draw the absorption depth when a photon is screened: the mean number of
