@@ -263,7 +263,7 @@ def stages_sample(local, photons=100_000_000, sources=1_000_000, shifts=64, reps
     ms = _event_ms(run, stream, reps, flush)
     acc = int(d_cnt.item())
     algo = 32 * nh + 56 * acc
-    be = {"hits": nh, "accepted": acc, "device_ms": ms, "hits_per_s": nh / (ms / 1e3), "gpu_launches": 3,
+    be = {"hits": nh, "accepted": acc, "device_ms": ms, "hits_per_s": nh / (ms / 1e3), "gpu_launches": 2,
           "roofline": {"bound": "hbm", "achieved": algo / (ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                        "frac": (algo / (ms / 1e3) / 1e9) / hbm if hbm else None,
                        "bytes": "32 B read per hit + 56 B written per accepted hit",
@@ -293,7 +293,7 @@ def stages_sample(local, photons=100_000_000, sources=1_000_000, shifts=64, reps
     torch.cuda.synchronize()
     ms = _event_ms(run, stream, reps, flush)
     lk = {"hits": nh, "shifts": shifts, "doms": L.info()["doms"], "blocks": L.info()["blocks"], "device_ms": ms,
-          "evals_per_s": shifts / (ms / 1e3), "hit_shifts_per_s": nh * shifts / (ms / 1e3), "gpu_launches": 3}
+          "evals_per_s": shifts / (ms / 1e3), "hit_shifts_per_s": nh * shifts / (ms / 1e3), "gpu_launches": 2}
     try:
         sys.path.insert(0, os.path.join(ROOT, "tests"))
         import oracle_util as O  # CPU baseline leg: the oracle restatement of llh.cxx
