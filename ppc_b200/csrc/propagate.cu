@@ -1085,7 +1085,9 @@ constexpr float kScreenU = 0.135f;
 constexpr uint64_t kScreenFrom = 3;  // photons per lane
 
 // The warps at work.  The longest photon of a launch takes some 400 steps, of 1.6 us for a
-// lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them.  So a launch with
+// lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them (when these lines were
+// drawn; the step is a third shorter since, and 4 instead of 6 photons per lane still take 7%
+// longer for 4.5e5).  So a launch with
 // fewer photons than kLanePhotons for each lane uses fewer warps on every SM, whose steps are
 // shorter: 1e5 photons 872 -> 844 us, 3e5 1038 -> 947, 6e5 1100 -> 1050, 1e6 (all warps) 1393;
 // with 13 per lane 3e5 take 1155 and 1e6 1426 us.  In hole ice the step is longer and depends
