@@ -3,11 +3,10 @@
 //                 per-hit streams as Engine::accept), then for each time shift the hit's bin
 //                 round((t + dt - t0) / lbin) and, when it lies in the DOM's window and
 //                 outside its errata windows, +1 on that bin's block (dat::fill, dat::join,
-//                 llh/llh.cxx:469-482, 614-621), in the block's own counters in shared
+//                 llh/llh.cxx:469-482, 614-621), in counters of the CTA's own in shared
 //                 memory.  Simulated hits on DOMs without observed pulses count toward the
 //                 no-hit total (cascade::ppc, llh/llh.cxx:1694-1700).
-//   k_llh_accept  when the counters of all shifts do not fit: the acceptance alone, once,
-//                 for k_llh_count to run over parts of the shifts.
+//   k_llh_count_global  the same where the counters do not fit there.
 //   k_llh_terms   one thread per (shift, block): llf (llh/llh.cxx:637-662) in FP64, a
 //                 fixed-order tree sum per CTA; the last CTA of a shift adds the CTA sums in
 //                 a fixed order, the no-hit term and divides by ndof (fllh,
@@ -34,17 +33,15 @@ struct LlhDevice {
   int32_t* block_dom = nullptr;
   double2* win = nullptr;
   // counters of an evaluation, cleared by one memset: the no-hit total, one ticket per shift,
-  // simulated counts [block][shift], and (norm) counts in the DOMs' windows [DOM][shift]
+  // simulated counts per (block, shift), and (norm) counts in the DOMs' windows per (DOM, shift)
   unsigned int* work = nullptr;
   double* partial = nullptr;         // [shift][CTA] sums of llf terms
   int* errors = nullptr;
   int ndt_cap = 0;
-  float2* list = nullptr;            // accepted hits (slot, time) of an evaluation in parts
-  uint64_t list_cap = 0;
   CallBuffers io;                    // host-pointer evaluations
   ~LlhDevice() {
     for (void* p : {(void*)dom_slot, (void*)doms, (void*)bin_block, (void*)block_dat, (void*)block_dom, (void*)win,
-                    (void*)work, (void*)partial, (void*)errors, (void*)list})
+                    (void*)work, (void*)partial, (void*)errors})
       if (p) cudaFree(p);
   }
 };
@@ -58,6 +55,12 @@ constexpr int kMaxNewton = 200;
 
 constexpr int kCountThreads = 1024;
 constexpr size_t kCountSmem = 192 << 10;  // shared memory of the counters of one CTA, at most
+// Counters that do not fit in one CTA's shared memory: up to this many per shift the shifts are
+// shared out over the CTAs (k_llh_count), from there on the counters are in global memory
+// (k_llh_count_global).  1.4e6 hits, 64 shifts: 2400 blocks (four parts) 215 and 229 us, with
+// half of the hits on one DOM 206 and 326; 4800 blocks (seven parts) 389 and 227, 368 and 332;
+// 5 shifts, 16000 blocks (two parts) 108 and 66.
+constexpr size_t kPartCounters = 3072;
 
 struct CountArgs {
   BackArgs A;
@@ -65,14 +68,12 @@ struct CountArgs {
   const LlhDom* doms;
   const int32_t* bin_block;
   const double2* win;
-  const float2* list;   // accepted hits instead of A's (evaluation in parts)
-  unsigned int* simc;   // [block][shift]
-  unsigned int* stot;   // [DOM][shift]
+  unsigned int* simc;   // [block][shift], from k_llh_count_global [shift][block]
+  unsigned int* stot;   // [DOM][shift], [shift][DOM]
   unsigned long long* nohit;
   double t0, lbin;
-  int nblocks, ndt, unh, norm;
-  int j0, nj;           // the part's shifts [j0, j0 + nj) of ndt
-  int smem;             // the counters are in shared memory
+  int nblocks, ndom, ndt, unh, norm;
+  int parts, step;      // k_llh_count: CTA c counts shifts [c % parts * step, + step) of ndt
   double dt[PPCB_LLH_MAX_SHIFTS];
 };
 
@@ -90,12 +91,6 @@ __device__ __forceinline__ BinnedHit llh_hit(const BackArgs& A, const int32_t* d
     h.t = o.t;
   }
   return h;
-}
-
-__global__ void __launch_bounds__(kThreads) k_llh_accept(BackArgs A, const int32_t* dom_slot, float2* list) {
-  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  const BinnedHit h = llh_hit(A, dom_slot, k);
-  if (k < A.n) list[k] = make_float2(__int_as_float(h.slot), h.t);
 }
 
 // The reference's bin of time t shifted by dt, relative to the DOM's window: in [0, n2 - n1)
@@ -130,51 +125,37 @@ struct __align__(16) SharedHit {
 // A thread accepts a hit; then the warp takes its accepted hits a few at a time, 2^k lanes
 // per hit and a lane per shift, so that the lanes have work whatever was accepted and the
 // counters of a hit's shifts lie side by side ([block][shift]: no bank conflicts, where
-// hits of one block in all lanes would queue for one counter).  What bounds it is
-// instruction issue: the acceptance (about 250 instructions per hit) and about 15 per
+// hits of one block in all lanes would queue for one counter).  Where the counters of all
+// shifts do not fit, the CTAs share the shifts out and each part accepts the hits for itself.
+// What bounds it is instruction issue: the acceptance (about 250 instructions per hit) and about 15 per
 // (accepted hit, shift), against 60 of one thread's loop with a double-precision division and
 // a global atomic each.  Whole evaluation, 1.38e6 hits (0.55e6 accepted): 64 shifts 222 ->
 // 58 us, 16 shifts 90 -> 43, 5 shifts 63 -> 41, one 50 -> 39.
-template <bool LIST>
 __global__ void __launch_bounds__(kCountThreads, 1) k_llh_count(const __grid_constant__ CountArgs F) {
-  extern __shared__ unsigned int cnt[];
+  extern __shared__ unsigned int cnt[];  // [block][shift], then with norm [DOM][shift]
   __shared__ unsigned int s_nohit;
   __shared__ double s_dt[PPCB_LLH_MAX_SHIFTS];
   __shared__ float s_q[PPCB_LLH_MAX_SHIFTS];
   const float inv = (float)(1 / F.lbin);
   __shared__ SharedHit s_hits[kCountThreads];
   SharedHit* mine = s_hits + (threadIdx.x & ~31);
-  const int group = F.nj > 16 ? 32 : F.nj > 8 ? 16 : F.nj > 4 ? 8 : F.nj > 1 ? 4 : 1;  // lanes per hit
-  const int counters = F.nblocks * F.nj;
-  if (F.smem)
-    for (int i = threadIdx.x; i < counters; i += kCountThreads) cnt[i] = 0;
+  const int part = blockIdx.x % F.parts, j0 = part * F.step, nj = min(F.step, F.ndt - j0);
+  const int group = nj > 16 ? 32 : nj > 8 ? 16 : nj > 4 ? 8 : nj > 1 ? 4 : 1;  // lanes per hit
+  const int sims = F.nblocks * nj, counters = sims + (F.norm ? F.ndom * nj : 0);
+  for (int i = threadIdx.x; i < counters; i += kCountThreads) cnt[i] = 0;
   if (threadIdx.x == 0) s_nohit = 0;
-  if (threadIdx.x < F.nj) {
-    s_dt[threadIdx.x] = F.dt[F.j0 + threadIdx.x];
+  if (threadIdx.x < nj) {
+    s_dt[threadIdx.x] = F.dt[j0 + threadIdx.x];
     s_q[threadIdx.x] = quot_part((float)s_dt[threadIdx.x] * inv);
   }
   __syncthreads();
   const unsigned int lane = threadIdx.x & 31;
   unsigned int nohit = 0;
-  auto add = [&](int bin, int base, int slot, int j) {
-    const int blk = F.bin_block[base + bin];
-    if (F.smem) atomicAdd(&cnt[blk * F.nj + j], 1u);
-    else atomicAdd(&F.simc[(size_t)blk * F.ndt + F.j0 + j], 1u);
-    if (F.norm) atomicAdd(&F.stot[(size_t)slot * F.ndt + F.j0 + j], 1u);  // only norm reads it
-  };
-  const uint64_t tiles = (F.A.n + 31) / 32, warps = (uint64_t)gridDim.x * (kCountThreads / 32);
-  for (uint64_t tile = (uint64_t)blockIdx.x * (kCountThreads / 32) + (threadIdx.x >> 5); tile < tiles; tile += warps) {
-    const uint64_t k = tile * 32 + lane;
-    BinnedHit h{-2, 0.f};
-    if constexpr (LIST) {
-      if (k < F.A.n) {
-        const float2 v = F.list[k];
-        h = BinnedHit{__float_as_int(v.x), v.y};
-      }
-    } else {
-      h = llh_hit(F.A, F.dom_slot, k);
-    }
-    if (F.unh && F.j0 == 0 && h.slot == -1) nohit++;
+  const uint64_t tiles = (F.A.n + 31) / 32, warps = (uint64_t)(gridDim.x / F.parts) * (kCountThreads / 32);
+  for (uint64_t tile = (uint64_t)(blockIdx.x / F.parts) * (kCountThreads / 32) + (threadIdx.x >> 5); tile < tiles;
+       tile += warps) {
+    const BinnedHit h = llh_hit(F.A, F.dom_slot, tile * 32 + lane);
+    if (F.unh && part == 0 && h.slot == -1) nohit++;
     const unsigned int m = __ballot_sync(0xffffffffu, h.slot >= 0);
     if (h.slot >= 0) {
       const LlhDom& D = F.doms[h.slot];
@@ -185,23 +166,62 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_llh_count(const __grid_con
     const int hits = __popc(m);
     for (int i = lane / group; i < hits; i += 32 / group) {
       const SharedHit x = mine[i];
-      for (int j = lane & (group - 1); j < F.nj; j += group) {
+      for (int j = lane & (group - 1); j < nj; j += group) {
         const int bin = llh_bin(F, x.q + s_q[j], x.t, s_dt[j], x.n1, x.n2, x.win0, x.nwin);
-        if ((unsigned)bin < (unsigned)(x.n2 - x.n1)) add(bin, x.base, x.slot, j);
+        if ((unsigned)bin < (unsigned)(x.n2 - x.n1)) {
+          atomicAdd(&cnt[F.bin_block[x.base + bin] * nj + j], 1u);
+          if (F.norm) atomicAdd(&cnt[sims + x.slot * nj + j], 1u);  // only norm reads it
+        }
       }
     }
     __syncwarp();
   }
   if (nohit) atomicAdd(&s_nohit, nohit);
   __syncthreads();
-  if (F.smem)
-    for (int i = threadIdx.x; i < counters; i += kCountThreads) {
-      const unsigned int c = cnt[i];
-      if (c) {
-        const int blk = i / F.nj;
-        atomicAdd(&F.simc[(size_t)blk * F.ndt + F.j0 + (i - blk * F.nj)], c);
-      }
+  for (int i = threadIdx.x; i < counters; i += kCountThreads) {
+    const unsigned int c = cnt[i];
+    const int b = i / nj, j = j0 + i - b * nj;  // the DOMs' counters follow the blocks'
+    if (c) atomicAdd(b < F.nblocks ? &F.simc[(size_t)b * F.ndt + j] : &F.stot[(size_t)(b - F.nblocks) * F.ndt + j], c);
+  }
+  if (threadIdx.x == 0 && s_nohit) atomicAdd(F.nohit, (unsigned long long)s_nohit);
+}
+
+// Where the counters do not fit in shared memory: a thread per hit, a loop over the shifts,
+// counters in global memory.  Bound by additions to the same counters, as hits crowd on a few
+// DOMs: lanes that add to one address at a time go out as one addition, and every warp starts
+// with another shift.  1.4e6 hits, 64 shifts, 16000 blocks: 240 us, with half of the hits on one
+// DOM 359 (a lane per shift, as above, 202 and 829).
+__global__ void __launch_bounds__(kThreads) k_llh_count_global(const __grid_constant__ CountArgs F) {
+  __shared__ unsigned int s_nohit;
+  __shared__ double s_dt[PPCB_LLH_MAX_SHIFTS];
+  __shared__ float s_q[PPCB_LLH_MAX_SHIFTS];
+  const float inv = (float)(1 / F.lbin);
+  if (threadIdx.x == 0) s_nohit = 0;
+  if (threadIdx.x < F.ndt) {
+    s_dt[threadIdx.x] = F.dt[threadIdx.x];
+    s_q[threadIdx.x] = quot_part((float)s_dt[threadIdx.x] * inv);
+  }
+  __syncthreads();
+  const BinnedHit h = llh_hit(F.A, F.dom_slot, (uint64_t)blockIdx.x * kThreads + threadIdx.x);
+  if (F.unh && h.slot == -1) atomicAdd(&s_nohit, 1u);
+  LlhDom D;
+  D.n1 = D.n2 = D.nwin = 0;  // no bin is taken
+  float q = 0;
+  if (h.slot >= 0) {
+    D = F.doms[h.slot];
+    q = quot_part((float)((double)h.t - F.t0) * inv);
+  }
+  int j = (int)((blockIdx.x * (kThreads / 32) + threadIdx.x / 32) % F.ndt);
+  for (int i = 0; i < F.ndt; i++, j = j + 1 < F.ndt ? j + 1 : 0) {
+    const int bin = llh_bin(F, q + s_q[j], h.t, s_dt[j], D.n1, D.n2, D.win0, D.nwin);
+    const bool in = (unsigned)bin < (unsigned)(D.n2 - D.n1);
+    __syncwarp();  // lanes that took either way of llh_bin add together
+    if (in) {
+      atomicAdd(&F.simc[(size_t)j * F.nblocks + F.bin_block[D.bin0 + bin]], 1u);
+      if (F.norm) atomicAdd(&F.stot[(size_t)j * F.ndom + h.slot], 1u);  // only norm reads it
     }
+  }
+  __syncthreads();
   if (threadIdx.x == 0 && s_nohit) atomicAdd(F.nohit, (unsigned long long)s_nohit);
 }
 
@@ -255,8 +275,8 @@ __device__ double cta_sum(double v, double* sh) {
 }
 
 struct TermArgs {
-  const unsigned int* simc;   // [block][shift]
-  const unsigned int* stot;   // [DOM][shift]
+  const unsigned int* simc;   // count of (block b, shift j): [b * block_step + j * shift_step]
+  const unsigned int* stot;   // of (DOM d, shift j): [d * block_step + j * dom_shift_step]
   const unsigned long long* nohit;
   unsigned int* ticket;       // [shift] CTAs done
   const double* block_dat;
@@ -266,7 +286,8 @@ struct TermArgs {
   int* errors;
   double* out;
   double nsim, ndat, sig;
-  int nblocks, ndom, ndt, norm, ndof;
+  int nblocks, ndt, norm, ndof;
+  int block_step, shift_step, dom_shift_step;
 };
 
 __global__ void __launch_bounds__(kThreads) k_llh_terms(TermArgs T) {
@@ -276,12 +297,12 @@ __global__ void __launch_bounds__(kThreads) k_llh_terms(TermArgs T) {
   double v = 0;
   bool err = false;
   if (b < T.nblocks) {
-    const double s = T.simc[(size_t)b * T.ndt + j];
+    const double s = T.simc[(size_t)b * T.block_step + (size_t)j * T.shift_step];
     double nsim = T.nsim;
     bool use = true;
     if (T.norm) {
       const int slot = T.block_dom[b];
-      const double st = T.stot[(size_t)slot * T.ndt + j];
+      const double st = T.stot[(size_t)slot * T.block_step + (size_t)j * T.dom_shift_step];
       if (st > 0) nsim = st * T.ndat / T.doms[slot].dtot;
       else use = false;  // dat::llh returns 0 for a DOM without simulated hits
     }
@@ -320,17 +341,15 @@ T* upload_vec(const std::vector<T>& v, const char* what) {
   return p;
 }
 
-// The counting kernels' shared-memory limit, once per device (a function attribute; before
-// any stream capture that launches them there).
+// The counting kernel's shared-memory limit, once per device (a function attribute; before
+// any stream capture that launches it there).
 void count_prepare() {
   static std::atomic<uint64_t> done{0};
   int dev = 0;
   check(cudaGetDevice(&dev), "cudaGetDevice");
   const uint64_t bit = 1ull << (dev & 63);
   if (done.load() & bit) return;
-  check(cudaFuncSetAttribute(k_llh_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem),
-        "likelihood attribute");
-  check(cudaFuncSetAttribute(k_llh_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem),
+  check(cudaFuncSetAttribute(k_llh_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem),
         "likelihood attribute");
   done.fetch_or(bit);
 }
@@ -373,7 +392,7 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   LlhDevice& D = *d_;
   const int nblocks = (int)blocks.size(), ndom = (int)doms.size();
   const int parts = std::max(1, (nblocks + kThreads - 1) / kThreads);
-  // the evaluation's counters: no-hit total, tickets, [block][shift], [DOM][shift] with norm
+  // the evaluation's counters: no-hit total, tickets, blocks x shifts, DOMs x shifts with norm
   const size_t ntick = (ndt + 1) / 2 * 2, nsimc = ((size_t)ndt * nblocks + 1) / 2 * 2;
   auto words = [&](int m) {
     return 2 + (size_t)(m + 1) / 2 * 2 + ((size_t)m * nblocks + 1) / 2 * 2 + (opts.norm ? (size_t)m * ndom : 0);
@@ -394,58 +413,43 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   unsigned int* simc = ticket + ntick;
   unsigned int* stot = simc + nsimc;
   check(cudaMemsetAsync(D.work, 0, words(ndt) * sizeof(unsigned int), st), "memset");
+  // where the counters are: with all shifts or a part of them in shared memory, or in global memory
+  const size_t per_shift = std::max(1, nblocks + (opts.norm ? ndom : 0));
+  const size_t parts_needed = (per_shift * ndt * sizeof(unsigned int) + kCountSmem - 1) / kCountSmem;
+  const bool fits = parts_needed == 1 || per_shift <= kPartCounters;
   if (n > 0) {
-    if ((n + kThreads - 1) / kThreads > 0x7fffffffull) throw Error("likelihood: too many hits in one call", 7);
+    const uint64_t grid = (n + kThreads - 1) / kThreads;
+    if (grid > 0x7fffffffull) throw Error("likelihood: too many hits in one call", 7);
     CountArgs F;
     F.A = back_args(eng_, dev_, dhits, n, seed);
     F.dom_slot = D.dom_slot;
     F.doms = D.doms;
     F.bin_block = D.bin_block;
     F.win = D.win;
-    F.list = nullptr;
     F.simc = simc;
     F.stot = stot;
     F.nohit = nohit;
     F.t0 = t0;
     F.lbin = lbin;
     F.nblocks = nblocks;
+    F.ndom = ndom;
     F.ndt = ndt;
     F.unh = opts.unh;
     F.norm = opts.norm;
     for (int j = 0; j < PPCB_LLH_MAX_SHIFTS; j++) F.dt[j] = j < ndt ? dts[j] : 0.0;
-    // shifts per pass: as many as have their counters in shared memory; when not even one
-    // shift's fit, all of them in one pass over counters in global memory
-    const size_t row = (size_t)std::max(1, nblocks) * sizeof(unsigned int);
-    F.smem = row <= kCountSmem;
-    const int step = F.smem ? (int)std::min<size_t>(ndt, kCountSmem / row) : ndt;
-    const size_t smem = F.smem ? (size_t)step * row : 0;
-    count_prepare();
-    // a CTA per SM, fewer when there are less than 256 hits for each: every CTA clears and
-    // adds up counters of its own (3e4 hits, 64 shifts: 45 us with 2048 hits per CTA)
-    const uint64_t sms = eng_.devs.at(dev_).prop.multiProcessorCount;
-    const unsigned int grid = (unsigned int)std::max<uint64_t>(1, std::min<uint64_t>(sms, (n + 255) / 256));
-    // more than one pass: the acceptance once, into a list kept between calls (a captured
-    // call cannot grow it and accepts in every pass instead)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (step < ndt && n > D.list_cap) check(cudaStreamIsCapturing(st, &cap), "capture status");
-    if (step < ndt && (n <= D.list_cap || cap == cudaStreamCaptureStatusNone)) {
-      if (n > D.list_cap) {
-        if (D.list) cudaFree(D.list);
-        D.list = nullptr;
-        D.list_cap = 0;
-        check(cudaMalloc((void**)&D.list, n * sizeof(float2)), "likelihood scratch");
-        D.list_cap = n;
-      }
-      k_llh_accept<<<(unsigned int)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(F.A, D.dom_slot, D.list);
-      check(cudaGetLastError(), "likelihood acceptance");
-      F.list = D.list;
+    if (fits) {
+      count_prepare();
+      F.step = (int)((ndt + parts_needed - 1) / parts_needed);
+      F.parts = (ndt + F.step - 1) / F.step;
+      // a CTA per SM, fewer when there are less than 256 hits for each: every CTA clears and
+      // adds up counters of its own (3e4 hits, 64 shifts: 45 us with 2048 hits per CTA)
+      const uint64_t sms = eng_.devs.at(dev_).prop.multiProcessorCount;
+      const unsigned int ctas = (unsigned int)std::max<uint64_t>(1, std::min(sms / F.parts, grid)) * F.parts;
+      k_llh_count<<<ctas, kCountThreads, F.step * per_shift * sizeof(unsigned int), st>>>(F);
+    } else {
+      k_llh_count_global<<<(unsigned int)grid, kThreads, 0, st>>>(F);
     }
-    for (F.j0 = 0; F.j0 < ndt; F.j0 += step) {
-      F.nj = std::min(step, ndt - F.j0);
-      if (F.list) k_llh_count<true><<<grid, kCountThreads, smem, st>>>(F);
-      else k_llh_count<false><<<grid, kCountThreads, smem, st>>>(F);
-      check(cudaGetLastError(), "likelihood count");
-    }
+    check(cudaGetLastError(), "likelihood count");
   }
   TermArgs T;
   T.simc = simc;
@@ -462,8 +466,10 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   T.ndat = opts.drep;
   T.sig = opts.sig;
   T.nblocks = nblocks;
-  T.ndom = ndom;
   T.ndt = ndt;
+  T.block_step = fits ? ndt : 1;
+  T.shift_step = fits ? 1 : nblocks;
+  T.dom_shift_step = fits ? 1 : ndom;
   T.norm = opts.norm;
   T.ndof = ndof;
   k_llh_terms<<<dim3(parts, ndt), kThreads, 0, st>>>(T);

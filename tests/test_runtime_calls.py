@@ -1,0 +1,79 @@
+"""What the library asks of the CUDA runtime, on a runtime without a GPU (fake_cudart.cpp):
+kernels and attributes inside stream captures, memory held between calls."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+from ppc_b200 import build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+HEAD = """
+import ctypes as C, json, sys
+sys.path.insert(0, {root!r})
+import numpy as np
+import ppc_b200._lib as native
+native.LIBPATH = {lib!r}
+from ppc_b200 import types as T, workloads as W
+from ppc_b200.api import PPC, Batch, Likelihood
+rt = C.CDLL({lib!r})
+rt.fake_log.restype = C.c_char_p
+rt.fake_pinned.restype = rt.fake_device.restype = C.c_size_t
+
+def log():
+    return rt.fake_log().decode().splitlines()
+
+def ctx(**opts):
+    c = PPC()
+    c.initialize(1.0, {ice!r})
+    c.set_seed(1)
+    c.set_options(**opts)
+    c.choose(0)
+    c.ini()
+    return c
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    build.build()
+    d = tmp_path_factory.mktemp("fake")
+    names = build.CU + [f"{f}.{k}" for f, k in build.PARTS] + build.CPP
+    objs = [os.path.join(build.OBJ, n + ".o") for n in names]
+    rt, lib = str(d / "fake_cudart.o"), str(d / "libppcb_fake.so")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "fake_cudart.cpp")
+    subprocess.run([build.CXX, "-std=c++17", "-O1", "-fPIC", "-I" + os.path.join(build.CUDA_HOME, "include"), "-c", src,
+                    "-o", rt], check=True)
+    subprocess.run([build.CXX, "-shared", "-Wl,-Bsymbolic", "-o", lib, rt] + objs, check=True)
+    return lib
+
+
+def _run(lib, ice, body):
+    """What `body` leaves in `result`, in a process of its own."""
+    code = HEAD.format(root=ROOT, lib=lib, ice=ice) + body + "\nprint('RESULT', json.dumps(result))\n"
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return json.loads(r.stdout.split("RESULT", 1)[1])
+
+
+@pytest.mark.parametrize("doms", [60, 400])
+def test_likelihood_scratch_does_not_follow_the_hits(fake, ice_full2d, doms):
+    """An evaluation's device memory is what the shifts need, whatever the number of hits: a
+    later call of more hits gives nothing back that a captured call would still write to."""
+    first, then = _run(fake, ice_full2d, """
+c = ctx()
+dom, per = np.repeat(np.arange(%d), 20), np.tile(np.arange(20), %d)
+d = np.zeros(len(dom), T.LLH_HIT_DTYPE)
+d["str"], d["om"], d["t"], d["q"] = dom // 60 + 1, dom %% 60 + 1, 100.0 + 50.0 * per, 20.0
+L = Likelihood(c, d, lbin=25.0)
+assert L.info()["blocks"] > 768  # 64 shifts' counters are more than one CTA's shared memory
+dts, h, out = np.linspace(-100, 100, 64), np.zeros(5000, T.HIT_DTYPE), np.zeros(64)
+result = []
+for n in (1000, 5000):
+    L.eval_device(h.ctypes.data, n, dts, 1.0, out.ctypes.data)
+    result.append(rt.fake_device())
+""" % (doms, doms))
+    assert first == then
