@@ -147,6 +147,7 @@ static void enqueue(Engine& eng, int d, cudaStream_t st, uint32_t maxE, uint32_t
 
 void Batch::capture() {
   release_graph();
+  check(propagate_prepare(eng_.args_for(d_), eng_.devs[d_].shape), "propagate attribute");
   cudaGraph_t g;
   check(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal), "begin capture");
   enqueue(eng_, d_, st_, maxE_, maxB_, hcap_, bunches_, bstart_, ev_off_, ev_cap_, ev_cnt_, dyn_, hits_, out_,
@@ -257,6 +258,7 @@ TuneResult Batch::autotune(const ppcb_bunch* b, int nb, uint32_t events, uint64_
     g.shape = keep;
     eng_.refill_below = keep_refill;
   }
+  eng_.prepare(d_);
   release_graph();  // kernel parameters changed: capture again on the next run
   return best;
 }

@@ -221,8 +221,18 @@ void Engine::ini() {
     check(cudaMallocHost((void**)&g.hhits, g.hhits_cap * sizeof(ppcb_hit)), "pinned hits");
   }
   inited_ = true;
+  for (size_t d = 0; d < devs.size(); d++) prepare((int)d);
   reset_streams();
   for (auto& g : devs) check(cudaStreamSynchronize(g.st), "sync");
+}
+
+void Engine::prepare(int d) {
+  check(cudaSetDevice(devs.at(d).dev), "cudaSetDevice");
+  KArgs a = args_for(d);
+  for (int mode : {0, 2}) {  // thread streams (1 takes the same kernel), per-photon streams
+    a.deterministic = mode;
+    check(propagate_prepare(a, devs[d].shape), "propagate attribute");
+  }
 }
 
 void Engine::reset_streams() {

@@ -183,6 +183,9 @@ class Engine {
   BackendTables& backend_tables(int d);
   double total_device_ms() const;
   KArgs args_for(int d) const;
+  // Sets the propagation kernels' attributes for the device's launch shape, so that a caller's
+  // capture finds them set.
+  void prepare(int d);
 
  private:
   void free_device(DeviceCtx& g);

@@ -317,8 +317,7 @@ GradGraph::GradGraph(Engine& e, const ppcb_bunch* b, int nb, uint32_t events, co
         "H2D");
   check(cudaStreamSynchronize(st), "gradient graph set-up");
 
-  // the recording kernel's shape (as Engine::gradient picks it); the occupancy queries also
-  // set the kernels' shared-memory attributes, which must happen before the capture
+  // the recording kernel's shape (as Engine::gradient picks it)
   KArgs a = e.args_for(0);
   a.bunches = S.bunches.p; a.bstart = S.bstart.p; a.nb = nb; a.num = S.photons;
   a.hits = S.hits.p; a.hcap = hit_cap; a.ctrl = S.ctrl.p; a.prov = S.prov.p;
@@ -333,6 +332,8 @@ GradGraph::GradGraph(Engine& e, const ppcb_bunch* b, int nb, uint32_t events, co
   KArgs r = e.args_for(0);
   r.ctrl = S.ctrl.p;
   const unsigned long long* nh_dev = &S.ctrl.p->hidx;
+  // the captured kernels' shared-memory attributes, before the capture
+  check(propagate_prepare(a, shape), "recording attribute");
   check(adjoint_prepare(r), "replay attribute");
 
   // the timing events are recorded as external event nodes, so that a replay records them

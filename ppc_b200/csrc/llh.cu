@@ -373,6 +373,7 @@ void Likelihood::upload() {
   D.win = upload_vec(w, "likelihood tables");
   check(cudaMalloc((void**)&D.errors, sizeof(int)), "likelihood scratch");
   check(cudaMemset(D.errors, 0, sizeof(int)), "likelihood scratch");
+  count_prepare();
 }
 
 Likelihood::~Likelihood() {
@@ -438,7 +439,6 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
     F.norm = opts.norm;
     for (int j = 0; j < PPCB_LLH_MAX_SHIFTS; j++) F.dt[j] = j < ndt ? dts[j] : 0.0;
     if (fits) {
-      count_prepare();
       F.step = (int)((ndt + parts_needed - 1) / parts_needed);
       F.parts = (ndt + F.step - 1) / F.step;
       // a CTA per SM, fewer when there are less than 256 hits for each: every CTA clears and

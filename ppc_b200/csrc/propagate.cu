@@ -1447,7 +1447,7 @@ cudaError_t model_adjoint(const KArgs& a, const ppcb_hit* hits, const void* prov
                           const float* wdom, const float2* wgrad, double* g_out, unsigned int* stats, int blocks,
                           cudaStream_t st, const unsigned long long* nh_dev);
 template <int MODEL>
-cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st);
+cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st, bool launch);
 template <int MODEL>
 cudaError_t model_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f, cudaStream_t st);
 template <int MODEL>
@@ -1508,7 +1508,12 @@ cudaError_t launch_dom_hist(const ppcb_hit* hits, uint64_t nh, unsigned int* cou
 
 cudaError_t launch_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st) {
   if (a.deterministic < 0 || a.deterministic > 2) return cudaErrorInvalidValue;
-  return with_model(a, [&](auto m) { return model_propagate<decltype(m)::value>(a, sh, st); });
+  return with_model(a, [&](auto m) { return model_propagate<decltype(m)::value>(a, sh, st, true); });
+}
+
+cudaError_t propagate_prepare(const KArgs& a, LaunchShape sh) {
+  if (a.deterministic < 0 || a.deterministic > 2) return cudaErrorInvalidValue;
+  return with_model(a, [&](auto m) { return model_propagate<decltype(m)::value>(a, sh, nullptr, false); });
 }
 
 // Phase-1 only: thread t samples photon t with stream t (test entry point).
@@ -1589,45 +1594,46 @@ __global__ void k_index_probe(const __grid_constant__ KArgs a, const float4* pos
 // static (deterministic = 1: thread streams, photon i on thread i mod T, nothing interleaves).
 // Dynamic shared memory: the photon pools (and provenance slots), then the
 // string-proximity cell entries; the attribute allows the largest table.
+// `launch` false: only the attribute is set.
 template <int BLOCK, int MINB, bool REC, bool STREAMS, int MODEL>
-static cudaError_t launch_one(const KArgs& a, int blocks, cudaStream_t st) {
+static cudaError_t launch_one(const KArgs& a, int blocks, cudaStream_t st, bool launch) {
   constexpr size_t dmax = dyn_smem<BLOCK, REC, STREAMS>() + kSgMaxCells * sizeof(uint16_t) + kBfrBytes;
   const size_t dyn = dyn_smem<BLOCK, REC, STREAMS>() + sg_cells_bytes(a) + kBfrBytes;
   if (dyn > dmax) return cudaErrorInvalidValue;
   static std::atomic<uint64_t> done{0};
   const cudaError_t e = allow_smem(done, k_propagate<BLOCK, MINB, REC, STREAMS, MODEL>, dmax);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !launch) return e;
   k_propagate<BLOCK, MINB, REC, STREAMS, MODEL><<<blocks, BLOCK, dyn, st>>>(a);
   return cudaGetLastError();
 }
 
 template <bool REC, bool STREAMS, int MODEL>
-static cudaError_t launch_shape(const KArgs& a, LaunchShape sh, cudaStream_t st) {
+static cudaError_t launch_shape(const KArgs& a, LaunchShape sh, cudaStream_t st, bool launch) {
   if constexpr (REC) {
     switch (sh.threads) {
-      case 256: return launch_one<256, 3, true, STREAMS, MODEL>(a, sh.blocks, st);
-      case 864: return launch_one<864, 1, true, STREAMS, MODEL>(a, sh.blocks, st);
+      case 256: return launch_one<256, 3, true, STREAMS, MODEL>(a, sh.blocks, st, launch);
+      case 864: return launch_one<864, 1, true, STREAMS, MODEL>(a, sh.blocks, st, launch);
       default: return cudaErrorInvalidConfiguration;
     }
   } else {
     switch (sh.threads) {
-      case 256: return launch_one<256, 3, false, STREAMS, MODEL>(a, sh.blocks, st);
-      case 128: return launch_one<128, 6, false, STREAMS, MODEL>(a, sh.blocks, st);
-      case 768: return launch_one<768, 1, false, STREAMS, MODEL>(a, sh.blocks, st);
-      case 864: return launch_one<864, 1, false, STREAMS, MODEL>(a, sh.blocks, st);
+      case 256: return launch_one<256, 3, false, STREAMS, MODEL>(a, sh.blocks, st, launch);
+      case 128: return launch_one<128, 6, false, STREAMS, MODEL>(a, sh.blocks, st, launch);
+      case 768: return launch_one<768, 1, false, STREAMS, MODEL>(a, sh.blocks, st, launch);
+      case 864: return launch_one<864, 1, false, STREAMS, MODEL>(a, sh.blocks, st, launch);
       default: return cudaErrorInvalidConfiguration;
     }
   }
 }
 
 template <int MODEL>
-cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st) {
+cudaError_t model_propagate(const KArgs& a, LaunchShape sh, cudaStream_t st, bool launch) {
   if (a.prov) {
-    return a.deterministic == 1 ? launch_shape<true, false, MODEL>(a, sh, st)
-                                : launch_shape<true, true, MODEL>(a, sh, st);
+    return a.deterministic == 1 ? launch_shape<true, false, MODEL>(a, sh, st, launch)
+                                : launch_shape<true, true, MODEL>(a, sh, st, launch);
   }
-  return a.deterministic == 2 ? launch_shape<false, true, MODEL>(a, sh, st)
-                              : launch_shape<false, false, MODEL>(a, sh, st);
+  return a.deterministic == 2 ? launch_shape<false, true, MODEL>(a, sh, st, launch)
+                              : launch_shape<false, false, MODEL>(a, sh, st, launch);
 }
 
 // The replay's static shared memory plus the string-proximity table exceed the default
@@ -1698,7 +1704,7 @@ int model_rec_blocks(int threads, bool streams) {
   template cudaError_t model_adjoint<M>(const KArgs&, const ppcb_hit*, const void*, uint64_t, uint32_t, const float*, \
                                         const float2*, double*, unsigned int*, int, cudaStream_t,                    \
                                         const unsigned long long*);                                                  \
-  template cudaError_t model_propagate<M>(const KArgs&, LaunchShape, cudaStream_t);                                  \
+  template cudaError_t model_propagate<M>(const KArgs&, LaunchShape, cudaStream_t, bool);                            \
   template cudaError_t model_index_probe<M>(const KArgs&, const float4*, int, int32_t*, float*, cudaStream_t);
 PPCB_MODEL_LAUNCHES(PPCB_TILT)
 #if PPCB_TILT < 3

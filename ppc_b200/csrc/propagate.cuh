@@ -65,6 +65,9 @@ struct LaunchShape {
 
 // Kernel entry points (defined in propagate.cu).
 cudaError_t launch_propagate(const KArgs& a, LaunchShape s, cudaStream_t st);
+// Sets the shared-memory limit of the kernel that launch_propagate would launch, and so loads
+// it, on the current device: before a capture of that launch.
+cudaError_t propagate_prepare(const KArgs& a, LaunchShape sh);
 cudaError_t launch_generate(const KArgs& a, LaunchShape s, void* pbuf_out, cudaStream_t st);
 cudaError_t launch_index_probe(const KArgs& a, const float4* pos, int n, int32_t* out_i, float* out_f,
                                cudaStream_t st);

@@ -59,6 +59,48 @@ def _run(lib, ice, body):
     return json.loads(r.stdout.split("RESULT", 1)[1])
 
 
+CAPTURES = {
+    "propagate": """
+buf, bs = np.zeros(1 << 20, np.uint8), np.array([0, 1000], np.uint64)
+st, graph = C.addressof(C.create_string_buffer(8)), C.c_void_p()
+rt.cudaStreamBeginCapture(C.c_void_p(st), 0)
+c.propagate_device(buf.ctypes.data, bs.ctypes.data, 1, 1000, buf.ctypes.data, 10, buf.ctypes.data, stream=st)
+rt.cudaStreamEndCapture(C.c_void_p(st), C.byref(graph))
+""",
+    "batch": """
+b = W.cascade([0, 0, -100], [0, 0, 1], 1000, q=0)
+Batch(c, 1, 1, 10000).run(b, 1)
+""",
+    "fit": """
+b = W.cascade([0, 0, -100], [0, 0, 1], 1000, q=0)
+c.gradient_graph(b, np.ones(c.info()["gsize"], np.float32), hit_cap=1000)
+""",
+    "likelihood": """
+d = np.zeros(1, T.LLH_HIT_DTYPE)
+d["str"], d["om"], d["t"], d["q"] = 1, 1, 100.0, 20.0
+L = Likelihood(c, d)
+h, out = np.zeros(100, T.HIT_DTYPE), np.zeros(1)
+st, graph = C.addressof(C.create_string_buffer(8)), C.c_void_p()
+rt.cudaStreamBeginCapture(C.c_void_p(st), 0)
+L.eval_device(h.ctypes.data, 100, [0.0], 1.0, out.ctypes.data, stream=st)
+rt.cudaStreamEndCapture(C.c_void_p(st), C.byref(graph))
+""",
+}
+
+
+@pytest.mark.parametrize("opts", [{}, {"deterministic": True}, {"photon_streams": True}],
+                         ids=["threads", "static", "photon_streams"])
+@pytest.mark.parametrize("what", list(CAPTURES))
+@pytest.mark.parametrize("kind", ["small_tilt", "full2d"])
+def test_attributes_are_set_before_a_capture(fake, what, kind, opts, request):
+    """A process's first call is a captured one: the kernels that it launches have their
+    shared-memory limits, and are loaded, before the capture begins."""
+    log = _run(fake, request.getfixturevalue("ice_" + kind), f"c = ctx(**{opts!r})" + CAPTURES[what]
+               + "result = log()")
+    assert any(x.startswith("captured ") for x in log)
+    assert not [x for x in log if x.startswith("attribute-in-capture")]
+
+
 @pytest.mark.parametrize("doms", [60, 400])
 def test_likelihood_scratch_does_not_follow_the_hits(fake, ice_full2d, doms):
     """An evaluation's device memory is what the shifts need, whatever the number of hits: a
