@@ -1406,7 +1406,7 @@ __global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_con
     hk.g_ba = gba;
     hk.prov_out = nullptr;
     hk.start = nullptr;
-    while (!hk.done && ph.TOT != 0 && ph.steps < a.max_steps) {
+    while (!hk.done && ph.TOT != 0 && ph.steps <= a.max_steps - 1u) {  // 0: no cap
       step<MODEL>(a, S, dt, ph, s, nan_steps, hk);
       ph.steps++;
     }
