@@ -1176,8 +1176,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
   // index in the static order and the last bunch found
   __shared__ uint64_t s_sidx[BLOCK];
   __shared__ int s_hint[BLOCK];
-  __shared__ uint32_t s_steps[BLOCK];  // steps of the thread's finished photons
-  s_steps[threadIdx.x] = 0;
+  __shared__ StepTotal s_steps[BLOCK];
+  s_steps[threadIdx.x].n = 0;
   s_sidx[threadIdx.x] = gt;
   s_hint[threadIdx.x] = 0;
   unsigned int nan_steps = 0;
@@ -1334,12 +1334,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
       }
       if (ph.TOT == 0) {  // (a 64-bit atomic of the block's count is a loop: 1.3% of the kernel)
         alive = false;
-        s_steps[threadIdx.x] += ph.steps;
+        s_steps[threadIdx.x].add(ph.steps);
       }
     }
   }
   if constexpr (!STREAMS) a.rs[gt] = (uint64_t)s.x | ((uint64_t)s.y << 32);
-  atomicAdd(&bsteps, (unsigned long long)s_steps[threadIdx.x]);
+  atomicAdd(&bsteps, s_steps[threadIdx.x].n);
   __syncthreads();
   if (threadIdx.x == 0) atomicAdd(&a.ctrl->steps, bsteps);
 }

@@ -63,6 +63,16 @@ struct LaunchShape {
   int threads;
 };
 
+// Steps of a thread's finished photons over a launch, which may last for hours: a thread of a
+// full grid takes 2^32 steps in about four.
+struct StepTotal {
+  unsigned long long n;
+#if defined(__CUDACC__)
+  __host__ __device__
+#endif
+  void add(uint32_t steps) { n += steps; }
+};
+
 // Kernel entry points (defined in propagate.cu).
 cudaError_t launch_propagate(const KArgs& a, LaunchShape s, cudaStream_t st);
 // Sets the shared-memory limit of the kernel that launch_propagate would launch, and so loads
