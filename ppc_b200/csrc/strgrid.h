@@ -100,7 +100,8 @@ PPCB_SG_HD float sg_float(uint32_t bits) {
 PPCB_SG_HD int sg_cell(const StrGridParams& g, float rx, float ry) {
 #if defined(__CUDA_ARCH__)
   const float u = __saturatef(fmaf(rx, g.su, g.ou)), v = __saturatef(fmaf(ry, g.sv, g.ov));  // NaN: 0
-  return __float_as_int(fmaf(v, g.cv, kSgMagic)) * g.nx + __float_as_int(fmaf(u, g.cu, kSgMagic)) + g.base;
+  return (int)(__float_as_uint(fmaf(v, g.cv, kSgMagic)) * (uint32_t)g.nx + __float_as_uint(fmaf(u, g.cu, kSgMagic)) +
+               (uint32_t)g.base);  // unsigned: kSgMagicBits (nx + 1) wraps around, base takes it off again
 #else
   const float fu = std::fma(rx, g.su, g.ou), fv = std::fma(ry, g.sv, g.ov);
   const float u = fu > 0 ? (fu < 1 ? fu : 1.f) : 0.f, v = fv > 0 ? (fv < 1 ? fv : 1.f) : 0.f;
