@@ -291,38 +291,15 @@ void Engine::fin() {
   inited_ = false;
 }
 
-// The 1-d cells over the inner radii lr[1..lnum-2] and a metre on either side: per cell the
-// only radius that may lie in it (infinity: none) and the number of the interval below it.
-// A cell is widened by a hundredth of itself for the rounding of a point's cell number.
 void Engine::tilt_tables(std::vector<float2>& cells) {
   const ppcb_params& p = cfg.p;
   tilt_ = TiltFast{0.f, 0.f, {0.f, 0.f}, 0};
-  cells.assign(kTiltCells, make_float2(INFINITY, 0.f));
+  cells.assign(kTiltCells, make_float2(0.f, 0.f));
+  if (p.tmod == 1) tilt_.on = tilt_cells(cfg.lr.data(), p.lnum, tilt_, cells.data());
   if (p.tmod == 2) {
     tilt_.on = tilt_recip_ok(p.mstp[0]) && tilt_recip_ok(p.mstp[1]);
     for (int i = 0; i < 2; i++) tilt_.rstep[i] = 1 / p.mstp[i];
   }
-  if (p.tmod != 1 || p.lnum < 2) return;
-  const auto& lr = cfg.lr;
-  for (int k = 1; k < p.lnum; k++)
-    if (!tilt_recip_ok(lr[k] - lr[k - 1])) return;
-  const double lo = p.lnum > 2 ? lr[1] - 1.0 : lr[0], hi = p.lnum > 2 ? lr[p.lnum - 2] + 1.0 : lr[1];
-  const double w = (hi - lo) / (kTiltCells - 1);
-  tilt_.scale = (float)(1 / (hi - lo));
-  tilt_.off = (float)(-lo / (hi - lo));
-  for (int c = 0; c < kTiltCells; c++) {
-    int below = 0, inside = 0;
-    for (int k = 1; k < p.lnum - 1; k++) {
-      if (c > 0 && lr[k] < lo + (c - 0.51) * w) below++;
-      else if (c == kTiltCells - 1 || lr[k] <= lo + (c + 0.51) * w) inside++;
-    }
-    if (inside > 1) return;
-    const int j = 1 + below;
-    float jf;
-    memcpy(&jf, &j, sizeof(jf));
-    cells[c] = make_float2(inside ? lr[j] : INFINITY, jf);
-  }
-  tilt_.on = 1;
 }
 
 KArgs Engine::args_for(int d) const {

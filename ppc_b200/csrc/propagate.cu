@@ -225,13 +225,8 @@ struct DevTilt {
   const ppcb_params& d;
   const float2* __restrict__ lpg;
   __device__ __forceinline__ int interval(float nr) const {
-    if constexpr (FAST) {
-      const float u = __saturatef(fmaf(nr, a.tf.scale, a.tf.off));
-      const float2 c = S.tcell[__float_as_int(fmaf(u, kTiltCells - 1.f, kSgMagic)) - kSgMagicBits];
-      return __float_as_int(c.y) + !(nr < c.x);
-    } else {
-      return tilt_interval(d.lnum, [this](int i) { return i ? S.span[i].y : S.span[1].x; }, nr);
-    }
+    if constexpr (FAST) return tilt_cell_interval(a.tf, S.tcell, nr);
+    else return tilt_interval(d.lnum, [this](int i) { return i ? S.span[i].y : S.span[1].x; }, nr);
   }
   __device__ __forceinline__ float4 span(int j) const { return S.span[j]; }
   __device__ __forceinline__ float rstep(int i) const { return a.tf.rstep[i]; }

@@ -12,7 +12,11 @@
 #pragma once
 #include <vector_types.h>
 
+#include <cmath>
+#include <cstring>
+
 #include "ppcb_types.h"
+#include "strgrid.h"
 
 #if defined(__CUDACC__)
 #define PPCB_HD __host__ __device__ __forceinline__
@@ -63,6 +67,8 @@ inline bool tilt_recip_ok(float b) { return b > 1e-6f && b < 1e6f; }
 // radii; on = 0 where a map does not allow it (a single map, steps out of range, radii closer
 // than a cell).  The 1-d interval of nr comes from cell round(clamp(nr scale + off, 0, 1) x
 // (kTiltCells - 1)), which holds the only radius that may lie in it and the interval below.
+// The cells are numbered from the outermost inwards (scale < 0): a NaN, which the clamp turns
+// into 0, falls into the outermost cell, and its interval is the last one, as in the search.
 constexpr int kTiltCells = 64;
 struct TiltFast {
   float scale, off;
@@ -83,6 +89,47 @@ PPCB_HD int tilt_interval(int lnum, const Radii& lr, float nr) {
     if (j >= PPCB_LMAX) j = PPCB_LMAX - 1;  // a single-map table would run off the end
   }
   return j;
+}
+
+// The same from the cells.
+PPCB_HD int tilt_cell_interval(const TiltFast& f, const float2* cells, float nr) {
+#if defined(__CUDA_ARCH__)
+  const float u = __saturatef(fmaf(nr, f.scale, f.off));  // NaN: 0
+  const float2 c = cells[__float_as_int(fmaf(u, kTiltCells - 1.f, kSgMagic)) - kSgMagicBits];
+  return __float_as_int(c.y) + !(nr < c.x);
+#else
+  const float v = std::fma(nr, f.scale, f.off), u = v > 0 ? (v < 1 ? v : 1.f) : 0.f;
+  const float2 c = cells[(int)(std::fma(u, kTiltCells - 1.f, kSgMagic) - kSgMagic)];
+  int j;
+  std::memcpy(&j, &c.y, sizeof(j));
+  return j + !(nr < c.x);
+#endif
+}
+
+// The cells over the inner radii lr[1..lnum-2] and a metre on either side: per cell the only
+// radius that may lie in it (none: infinity, in the outermost cell minus infinity) and the
+// interval below it.  A cell is widened by a hundredth of itself for the rounding of a point's
+// cell number.  False where the map does not allow it.
+inline bool tilt_cells(const float* lr, int lnum, TiltFast& f, float2* cells) {
+  if (lnum < 2) return false;
+  for (int k = 1; k < lnum; k++)
+    if (!tilt_recip_ok(lr[k] - lr[k - 1])) return false;
+  const double lo = lnum > 2 ? lr[1] - 1.0 : lr[0], hi = lnum > 2 ? lr[lnum - 2] + 1.0 : lr[1];
+  const double w = (hi - lo) / (kTiltCells - 1);
+  f.scale = (float)(-1 / (hi - lo));
+  f.off = (float)(hi / (hi - lo));
+  for (int c = 0; c < kTiltCells; c++) {
+    int below = 0, inside = 0;
+    for (int k = 1; k < lnum - 1; k++) {
+      if (c < kTiltCells - 1 && lr[k] < hi - (c + 0.51) * w) below++;
+      else if (c == 0 || lr[k] <= hi - (c - 0.51) * w) inside++;
+    }
+    if (inside > 1) return false;
+    const int j = inside || c > 0 ? 1 + below : below;
+    std::memcpy(&cells[c].y, &j, sizeof(j));
+    cells[c].x = inside ? lr[j] : c > 0 ? INFINITY : -INFINITY;
+  }
+  return true;
 }
 
 // 1-d: interpolate between the two maps bracketing the distance along 225 deg

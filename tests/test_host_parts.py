@@ -2,6 +2,8 @@
 import os
 import subprocess
 
+import pytest
+
 from ppc_b200 import build
 
 
@@ -64,3 +66,52 @@ int main() {
 """, "-fsanitize=signed-integer-overflow", "-fsanitize-undefined-trap-on-error")
     bad, n = map(int, out.split())
     assert bad == 0 and n > 60_000
+
+
+@pytest.mark.parametrize("reach,spacing", [("2000", "uni(0, 2.5)")], ids=["detector"])
+def test_tilt_cells_give_the_interval_of_the_search(tmp_path, reach, spacing):
+    """The 1-d tilt interval from the cells (the kernel's expressions, on the host) against the
+    search among the radii: on the radii and a few ulps from them, on the cells' edges, far outside,
+    for infinities and NaN.  Maps of 2 to 79 radii from up to `reach` m, 10^spacing m apart."""
+    out = _run(tmp_path, """
+#include <cstdio>
+#include <random>
+#include "tilt.h"
+using namespace ppcb;
+int main() {
+  std::mt19937 g(5);
+  auto uni = [&](double a, double b) { return std::uniform_real_distribution<double>(a, b)(g); };
+  long bad = 0, points = 0, maps = 0, refused = 0;
+  for (int m = 0; m < 4000; m++) {
+    const int lnum = m % 4 == 0 ? 2 : m % 4 == 1 ? 3 : std::uniform_int_distribution<int>(4, 79)(g);
+    float lr[PPCB_LMAX] = {0};
+    lr[0] = (float)(uni(-1, 1) * REACH);
+    const double step = std::pow(10., SPACING);
+    for (int k = 1; k < lnum; k++) lr[k] = (float)(lr[k - 1] + step * uni(0.9, 1.1));
+    TiltFast f{};
+    float2 cells[kTiltCells];
+    if (!tilt_cells(lr, lnum, f, cells)) {
+      refused++;
+      continue;
+    }
+    maps++;
+    auto check = [&](float nr) {
+      points++;
+      bad += tilt_cell_interval(f, cells, nr) != tilt_interval(lnum, [&](int i) { return lr[i]; }, nr);
+    };
+    for (float x : {INFINITY, -INFINITY, NAN, 1e30f, -1e30f, 3e38f, -3e38f, 0.f}) check(x);
+    for (int k = 0; k < lnum; k++) {
+      float a = lr[k], b = lr[k];
+      for (int i = 0; i < 8; i++, a = std::nextafterf(a, INFINITY), b = std::nextafterf(b, -INFINITY)) check(a), check(b);
+    }
+    for (int c = -2; c < 2 * kTiltCells + 2; c++) {  // the cells' edges and centres
+      const float x = (float)((f.off - c / (2.0 * (kTiltCells - 1))) / -f.scale);
+      check(x), check(std::nextafterf(x, INFINITY)), check(std::nextafterf(x, -INFINITY));
+    }
+    for (int i = 0; i < 300; i++) check((float)uni(lr[0] - step, lr[lnum - 1] + step));
+  }
+  printf("%ld %ld %ld %ld", bad, points, maps, refused);
+}
+""", "-DREACH=" + reach, "-DSPACING=" + spacing)
+    bad, points, maps, refused = map(int, out.split())
+    assert bad == 0 and maps > 2000 and points > 1_000_000 and refused > 0, out

@@ -149,3 +149,25 @@ def test_models_propagate_alike(ice_full, tmp_path):
     np.testing.assert_allclose(r1["g_be"], r2["g_be"], rtol=1e-6, atol=1e-9 * np.abs(r1["g_be"]).max())
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("name", ["six", "two", "forty"])
+def test_1d_tilt_at_points_that_are_not_finite(ice_full, tmp_path, name, monkeypatch):
+    """NaN, infinite and huge positions give the general kernel's tilt shift."""
+    import torch
+    ice, rng, got = _tilted(ice_full, tmp_path / "ice", RADII[name]), np.random.default_rng(9), []
+    xy = rng.choice([np.nan, np.inf, -np.inf, 3e38, -3e38, 1.0], (4096, 2))
+    for vthk in (0, 1):
+        monkeypatch.setenv("VTHK", str(vthk))
+        c = _ctx(ice)
+        pos = _points(c, 4096, np.random.default_rng(9))
+        pos[:, :2] = xy
+        oi = torch.zeros((4096, 8), dtype=torch.int32, device="cuda")
+        of = torch.zeros((4096, 2), dtype=torch.float32, device="cuda")
+        d = torch.from_numpy(pos).cuda()
+        c.index_probe_device(d.data_ptr(), 4096, oi.data_ptr(), of.data_ptr())
+        torch.cuda.synchronize()
+        got.append(of.cpu().numpy()[:, 0])
+        c.close()
+    np.testing.assert_array_equal(got[0], got[1])  # NaN where it is NaN
+    assert np.isfinite(got[1]).any() and np.isnan(got[1]).any()
