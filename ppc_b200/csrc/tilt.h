@@ -116,6 +116,9 @@ inline bool tilt_cells(const float* lr, int lnum, TiltFast& f, float2* cells) {
     if (!tilt_recip_ok(lr[k] - lr[k - 1])) return false;
   const double lo = lnum > 2 ? lr[1] - 1.0 : lr[0], hi = lnum > 2 ? lr[lnum - 2] + 1.0 : lr[1];
   const double w = (hi - lo) / (kTiltCells - 1);
+  // a point's cell number is off by less than 63 (2 |off| + 2) / 2^24 of a cell, which has to be
+  // within a hundredth
+  if (std::fmax(std::fabs(lo), std::fabs(hi)) > 1000 * (hi - lo)) return false;
   f.scale = (float)(-1 / (hi - lo));
   f.off = (float)(hi / (hi - lo));
   for (int c = 0; c < kTiltCells; c++) {

@@ -68,7 +68,8 @@ int main() {
     assert bad == 0 and n > 60_000
 
 
-@pytest.mark.parametrize("reach,spacing", [("2000", "uni(0, 2.5)")], ids=["detector"])
+@pytest.mark.parametrize("reach,spacing", [("2000", "uni(0, 2.5)"), ("std::pow(10., uni(1, 6))", "uni(-1, 2.5)")],
+                         ids=["detector", "far"])
 def test_tilt_cells_give_the_interval_of_the_search(tmp_path, reach, spacing):
     """The 1-d tilt interval from the cells (the kernel's expressions, on the host) against the
     search among the radii: on the radii and a few ulps from them, on the cells' edges, far outside,
