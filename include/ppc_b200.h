@@ -10,6 +10,12 @@
  * globals (tables, device buffers, pending bunches, segment list, hit map), so several
  * contexts may coexist in one process; one context must not be used from two host
  * threads at once.  The record types are in ppc_b200/csrc/ppcb_types.h.
+ *
+ * Memory kept between calls: the entry points with host buffers (ppcb_accept, ppcb_sources,
+ * ppcb_llh_eval) keep up to four device buffers of at most 256 MB each per context and two per
+ * ppcb_llh, and 8 MB of pinned memory each; ppcb_gradient keeps device buffers of its largest
+ * call and two pinned ones of at most 16 MB.  ppcb_fin gives a context's back, and
+ * ppcb_llh_destroy a likelihood's.
  */
 #ifndef PPC_B200_H
 #define PPC_B200_H

@@ -44,6 +44,12 @@ struct DBuf {
 
 constexpr int kWBlocks = 592, kWThreads = 256;
 
+// Bins up to which a call's charges and counts go through pinned buffers that are kept (16 MB
+// each).  More are copied from and to pageable memory, which is no slower then: 3.1e6 bins 9.2
+// ms with the buffers and 10.9 without, 5.2e6 15.5 and 16.1, 15e6 48.8 and 46.7; the call that
+// pins the buffers 26-46 and 14, 45-70 and 20, 114-139 and 52.
+constexpr size_t kPinnedBins = 4u << 20;
+
 // Poisson weights w_d = scale (k_d / mu_d - 1) and the log-likelihood terms k_d log mu_d - mu_d
 // of the bins with mu_d = scale x simulated count > 0, summed per block in a fixed order
 // (strided per thread, then a tree).
@@ -158,7 +164,9 @@ Engine::Grad Engine::gradient(const ppcb_bunch* b, int nb, uint32_t events, cons
   X.wgrad.need(PPCB_WNUM);
   X.g.need(2 * PPCB_MAXLYS);
   X.stats.need(2);
-  X.hbins.need(nbins); X.hcounts.need(nbins); X.hstats.need(2); X.hg.need(2 * PPCB_MAXLYS); X.hctrl.need(1);
+  const bool pinned = nbins <= kPinnedBins;
+  if (pinned) { X.hbins.need(nbins); X.hcounts.need(nbins); }
+  X.hstats.need(2); X.hg.need(2 * PPCB_MAXLYS); X.hctrl.need(1);
   if (observed) { X.observed.need(nbins); X.part.need(kWBlocks); X.ll.need(1); X.hll.need(1); }
   auto& db = X.bunches;
   auto& dbs = X.bstart;
@@ -203,17 +211,20 @@ Engine::Grad Engine::gradient(const ppcb_bunch* b, int nb, uint32_t events, cons
   // through the host and back took 1.4 ms more, 72 hits of 4 events 0.95 ms)
   const unsigned long long* nh_dev = &dctrl.p->hidx;
   check(launch_dom_hist(dh.p, hit_cap, dcnt.p, events, gsize, st, nh_dev), "histogram");
+  std::vector<float> large(pinned || observed ? 0 : nbins);  // a call's weights beyond kPinnedBins
   if (observed) {
-    memcpy(X.hbins.p, observed, nbins * sizeof(float));
-    check(cudaMemcpyAsync(X.observed.p, X.hbins.p, nbins * sizeof(float), cudaMemcpyHostToDevice, st), "H2D charges");
+    if (pinned) memcpy(X.hbins.p, observed, nbins * sizeof(float));
+    check(cudaMemcpyAsync(X.observed.p, pinned ? X.hbins.p : observed, nbins * sizeof(float), cudaMemcpyHostToDevice,
+                          st), "H2D charges");
     k_weights<<<kWBlocks, kWThreads, 0, st>>>(dcnt.p, X.observed.p, nbins, scale, dw.p, X.part.p);
     check(cudaGetLastError(), "weights");
     k_ll_sum<<<1, kWThreads, 0, st>>>(X.part.p, kWBlocks, X.ll.p);
     check(cudaGetLastError(), "log-likelihood");
     check(cudaMemcpyAsync(X.hll.p, X.ll.p, sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
   } else {
-    for (size_t d = 0; d < nbins; d++) X.hbins.p[d] = (float)(scale * weights[d]);
-    check(cudaMemcpyAsync(dw.p, X.hbins.p, nbins * sizeof(float), cudaMemcpyHostToDevice, st), "H2D weights");
+    float* w = pinned ? X.hbins.p : large.data();
+    for (size_t d = 0; d < nbins; d++) w[d] = (float)(scale * weights[d]);
+    check(cudaMemcpyAsync(dw.p, w, nbins * sizeof(float), cudaMemcpyHostToDevice, st), "H2D weights");
   }
   // replay of the detected photons
   KArgs r = args_for(0);
@@ -221,7 +232,10 @@ Engine::Grad Engine::gradient(const ppcb_bunch* b, int nb, uint32_t events, cons
   check(launch_adjoint(r, dh.p, dprov.p, hit_cap, events, dw.p, dwg.p, dgo.p, dstat.p, adjoint_blocks(g.prop), st,
                        nh_dev), "replay launch");
   check(cudaEventRecord(e2, st), "event");
-  check(cudaMemcpyAsync(X.hcounts.p, dcnt.p, nbins * sizeof(unsigned int), cudaMemcpyDeviceToHost, st), "D2H");
+  Grad out;
+  if (!pinned) out.counts.resize(nbins);
+  check(cudaMemcpyAsync(pinned ? X.hcounts.p : out.counts.data(), dcnt.p, nbins * sizeof(unsigned int),
+                        cudaMemcpyDeviceToHost, st), "D2H");
   check(cudaMemcpyAsync(X.hg.p, dgo.p, 2 * PPCB_MAXLYS * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H gradient");
   check(cudaMemcpyAsync(X.hstats.p, dstat.p, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st), "D2H stats");
   check(cudaMemcpyAsync(X.hctrl.p, dctrl.p, sizeof(ppcb_ctrl), cudaMemcpyDeviceToHost, st), "D2H ctrl");
@@ -229,8 +243,7 @@ Engine::Grad Engine::gradient(const ppcb_bunch* b, int nb, uint32_t events, cons
   const ppcb_ctrl c = *X.hctrl.p;
   if (c.hidx > hit_cap) throw Error("gradient: hit capacity too small (" + std::to_string(c.hidx) + " hits)", 7);
   const uint64_t nh = c.hidx;
-  Grad out;
-  out.counts.assign(X.hcounts.p, X.hcounts.p + nbins);
+  if (pinned) out.counts.assign(X.hcounts.p, X.hcounts.p + nbins);
   out.ll = 0;
   if (observed) out.ll = *X.hll.p;
   const double* go = X.hg.p;

@@ -119,3 +119,20 @@ for n in (1000, 5000):
     result.append(rt.fake_device())
 """ % (doms, doms))
     assert first == then
+
+
+@pytest.mark.parametrize("given", ["observed", "weights"])
+def test_gradient_keeps_little_pinned_memory(fake, ice_small, given):
+    """Charges and counts of very many events do not stay behind in pinned memory."""
+    few, many, counts = _run(fake, ice_small, """
+c = ctx()
+gsize = c.info()["gsize"]
+b = W.cascade([0, 0, -100], [0, 0, 1], 1000, q=0)
+result = []
+for events in (64, 40 * (16 << 20) // (10 * gsize)):
+    n = events * gsize
+    r = c.gradient(b, events=events, %s=np.ones(n, np.float32), hit_cap=1000)
+    result.append(rt.fake_pinned())
+result.append(int(r["counts"].sum()))
+""" % given)
+    assert many - few <= 32 << 20 and counts == 0
