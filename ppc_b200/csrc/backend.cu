@@ -171,7 +171,8 @@ BackArgs back_args(Engine& e, int d, const ppcb_hit* dhits, uint64_t n, uint32_t
   BackendTables& T = e.backend_tables(d);
   const DeviceCtx& g = e.devs.at(d);
   BackArgs A;
-  A.hits = dhits; A.n = n; A.doms = T.doms; A.keys = T.keys; A.sensors = T.sensors; A.rat = T.rat; A.wvs = T.wvs; A.dirs = T.dirs;
+  A.hits = dhits; A.n = n;
+  A.doms = T.doms; A.keys = T.keys; A.sensors = T.sensors; A.rat = T.rat; A.wvs = T.wvs; A.dirs = T.dirs;
   A.rm = g.rm; A.nmul = (uint32_t)std::max(1, std::min(g.T, 1024)); A.seed = seed; A.gsize = e.cfg.p.gsize;
   A.wide = reinterpret_cast<uintptr_t>(dhits) % 32 == 0;
   return A;

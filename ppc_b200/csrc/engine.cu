@@ -255,8 +255,8 @@ void Engine::free_device(DeviceCtx& g) {
   g.io.reset();
   if (g.st) cudaStreamSynchronize(g.st);
   if (g.cp) cudaStreamSynchronize(g.cp);
-  void* ptrs[] = {g.absca, g.wmeta, g.lp, g.oms, g.az, g.sc, g.lr, g.ls, g.is, g.mcol, g.bfrt, g.sg_groups, g.sg_cells, g.tcell,
-                  g.rs, g.rm};
+  void* ptrs[] = {g.absca, g.wmeta, g.lp, g.oms, g.az, g.sc, g.lr, g.ls, g.is, g.mcol, g.bfrt, g.sg_groups, g.sg_cells,
+                  g.tcell, g.rs, g.rm};
   for (void* p : ptrs) if (p) cudaFree(p);
   g.absca = nullptr; g.wmeta = nullptr; g.lp = nullptr; g.oms = nullptr; g.az = nullptr; g.sc = nullptr;
   g.bfrt = nullptr; g.tcell = nullptr; g.sg_groups = nullptr; g.sg_cells = nullptr;

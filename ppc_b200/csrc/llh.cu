@@ -95,9 +95,10 @@ __device__ __forceinline__ BinnedHit llh_hit(const BackArgs& A, const int32_t* d
 
 // The reference's bin of time t shifted by dt, relative to the DOM's window: in [0, n2 - n1)
 // when the hit takes part.  `q` is the quotient in single precision, a sum of two numbers
-// below kMaxQuot (or a NaN), so within 1.5e-3 of it: at least 2e-3 from the middle between
-// two bins it decides; otherwise, and always with errata windows, the double-precision
-// expressions of llh/llh.cxx:469-482 do.
+// below kMaxQuot (or a NaN): each of them carries three roundings (operand, 1 / lbin, product;
+// 7.2e-4), their sum one more (2.4e-4), so q is within 1.7e-3 of it.  At least 2e-3 from the
+// middle between two bins it decides; otherwise, and always with errata windows, the
+// double-precision expressions of llh/llh.cxx:469-482 do.
 constexpr float kMaxQuot = 4000.f;
 __device__ __forceinline__ float quot_part(float q) { return fabsf(q) < kMaxQuot ? q : __int_as_float(0x7fffffff); }
 

@@ -601,7 +601,8 @@ struct Truncated {
 
 // gpu/pro.cu:677-717: a step cut short at fin (DOM hit or hole-ice entry): the optical
 // depths used over the bulk-ice part by layers, then the hole-ice part.
-static __device__ __noinline__ Truncated truncated_step(const ppcb_params& e, const float2* __restrict__ wz, float z, float nz,
+static __device__ __noinline__ Truncated truncated_step(const ppcb_params& e, const float2* __restrict__ wz, float z,
+                                                 float nz,
                                                  float fin, float edh, int I, int sign, float anz, float SCA,
                                                  float TOT, float nr, float hi, float hf, float del, float sca,
                                                  int om) {
@@ -686,7 +687,8 @@ __device__ __forceinline__ Found dom_search(const KArgs& a, const SmemTables& S,
   {  // DOM search, gpu/pro.cu:577-672
     int xlx, xhx, xly, xhy;
     cell_range(e, r.x, r.y, fa(r.x, fm(sca, n.x)), fa(r.y, fm(sca, n.y)), xlx, xhx, xly, xhy);
-    const bool hole_on = !plain(MODEL) && e.hr > 0 && (e.hifl == 0 || (e.hifl < 0 && r.w < -e.hifl) || (e.hifl > 0 && r.w > e.hifl));
+    const bool hole_on = !plain(MODEL) && e.hr > 0 &&
+                         (e.hifl == 0 || (e.hifl < 0 && r.w < -e.hifl) || (e.hifl > 0 && r.w > e.hifl));
     for (int i = xlx, j = xly; i <= xhx && j <= xhy; (++j <= xhy) ? 0 : (j = xly, i++)) {
       for (unsigned int k = S.is[i * PPCB_CY + j]; k != 0x8000;) {
         unsigned int m = S.ls[k];
@@ -879,7 +881,10 @@ __device__ __forceinline__ void step(const KArgs& a, const SmemTables& S, const 
         ra = h * aI.ra + g * aJ.ra;
         rb = h * aI.rb + g * aJ.rb;
         if ((unsigned)(I - J + 1) > 2u)
-          for (int i = I + sign; i != J && (unsigned)i < (unsigned)e.size; i += sign) { ra += S.az[i].ra; rb += S.az[i].rb; }
+          for (int i = I + sign; i != J && (unsigned)i < (unsigned)e.size; i += sign) {
+            ra += S.az[i].ra;
+            rb += S.az[i].rb;
+          }
         float f = edh / anz;
         ra *= f; rb *= f;
         ra = I == J ? q.x : ra;
@@ -1064,37 +1069,36 @@ struct PhotonPool {
 
 // The order in which a warp takes photons.  A photon's number of steps goes with its
 // absorption depth -log(u), so it is exponential: taken in index order, the last photons of
-// a launch leave the GPU with ever fewer live lanes for some ten mean lifetimes (350 steps
-// of 1.6-2.2 us each, 0.75 ms: half of the time of a launch of 1e6 photons).  So the first
-// photons, up to kScreenGroups per thread, are screened: a warp samples a group of 32 and at
-// once runs those with u < kScreenU (absorption depth above 2: 13.5% of them), and leaves the
-// others (a bit mask per group) to the end of the launch, when only short photons should
-// start.  Sampling a group takes the issue slots of about one step, so a screened photon,
-// sampled twice, costs 1/26 more.  Measured on the full detector's cascades without and with
-// it: 6e5 photons 1220 and 1104 us, 1e6 1634 and 1394, 3e6 3254 and 2776, 3e7 25810 and
-// 24970; 8 and 24 groups take 7% and 2% longer for 3e6, a kScreenU of 0.05 or 0.30 3% and 6%.
-// Below three photons per lane the launch lasts as long as its longest photon whenever that
-// starts, and nothing is screened.
+// a launch leave the GPU with ever fewer live lanes for some ten mean lifetimes (350 steps one
+// after the other).  So the first photons, up to kScreenGroups per thread, are screened: a warp
+// samples a group of 32 and at once runs those with u < kScreenU (absorption depth above 2:
+// 13.5% of them), and leaves the others (a bit mask per group) to the end of the launch, when
+// only short photons should start.  Sampling a group takes the issue slots of about one step, so
+// a screened photon, sampled twice, costs 1/26 more.  The full detector's cascades without and
+// with it: 3e5 photons 805 and 700 us, 6e5 971 and 818, 1e6 1316 and 1127, 3e6 2647 and 2302, 3e7
+// 20990 and 20650.  8 and 24 groups take 5% and 2.5% longer for 3e6; a kScreenU of 0.05 or 0.30
+// takes 3% and 3.5% (1e6: 2% and 7%).  Below three photons per lane the launch lasts as long as
+// its longest photon whenever that starts, and nothing is screened.
 constexpr int kScreenGroups = 16;
 constexpr float kScreenU = 0.135f;
 constexpr uint64_t kScreenFrom = 3;  // photons per lane
 
-// The warps at work.  The longest photon of a launch takes some 400 steps, of 1.6 us for a
-// lane alone, 2.0 us with five warps on the SM and 3.6 us with all of them (when these lines were
-// drawn; the step is a third shorter since, and 4 instead of 6 photons per lane still take 7%
-// longer for 4.5e5).  So a launch with
-// fewer photons than kLanePhotons for each lane uses fewer warps on every SM, whose steps are
-// shorter: 1e5 photons 872 -> 844 us, 3e5 1038 -> 947, 6e5 1100 -> 1050, 1e6 (all warps) 1393;
-// with 13 per lane 3e5 take 1155 and 1e6 1426 us.  In hole ice the step is longer and depends
-// less on the warps beside it, so there kLanePhotonsHole holds (a point source in the column
-// with 2 and with 6 per lane: 1.2e5 photons 687 and 864 us, 4e5 958 and 1064; without hole ice
-// 4e5 836 and 764).  Fewer photons than kFewWarps sixteenths of
-// the warps (five per SM) have lanes are dealt out over those warps at the start, a few lanes
-// each: 1000 photons 384 -> 283 us, 4096 630 -> 498, 3e4 785 -> 674 (five sixteenths: +4%).
+// The warps at work.  The longest photon of a launch takes some 400 steps, and a step takes more
+// than twice as long with all warps of the SM at work as for a lane alone.  So a launch with
+// fewer photons than kLanePhotons for each lane uses fewer warps on every SM.  With 2, 4, 6, 8
+// and 13 per lane 3e5 photons take 830, 700, 703, 702 and 844 us, 4.5e5 819, 794, 739, 743 and 841,
+// 6e5 876, 872, 816, 800 and 896, a flasher's 4e5 966, 983, 898, 982 and 1237, a muon's 1e6 1165,
+// 1162, 1158, 1251 and 1285.  In hole ice the step is longer and depends less on the warps
+// beside it, so there kLanePhotonsHole holds: a point source in the column with 1, 2, 4 and 6 per
+// lane 1.2e5 photons 660, 657, 772 and 797 us, 2e5 769, 749, 806 and 902, 4e5 963, 960, 1031 and
+// 1048.  Fewer photons than kFewWarps sixteenths of the warps (five per SM) have lanes are dealt
+// out over those warps at the start, a few lanes each: 3e4 photons 487 us, over five sixteenths
+// 504, over all warps 599.
 constexpr uint32_t kFewWarps = 3;
 constexpr uint64_t kLanePhotons = 6, kLanePhotonsHole = 2;
 
-// A warp's place in that order (shared memory; read and written by lane 0's turn only).
+// A warp's place in that order (shared memory; read by all lanes, written by lane 0 between the
+// two __syncwarp of a turn).
 struct WarpClaims {
   uint32_t left[kScreenGroups];  // screened groups: the lanes whose photon is left for the end
   int screened, finished;        // groups screened; groups whose left-over photons were taken
@@ -1139,7 +1143,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_propagate(const __grid_constant
     const uint32_t warps = gridDim.x * (BLOCK / 32), few = max(1u, warps * kFewWarps / 16);
     plan.num = num;
     plan.nb = a.dyn ? (int)a.dyn[1] : a.nb;
-    plan.warps = (uint32_t)max((uint64_t)few, min((uint64_t)warps, num / (32 * (!plain(MODEL) && a.p.hr > 0 ? kLanePhotonsHole : kLanePhotons))));
+    const uint64_t per_lane = !plain(MODEL) && a.p.hr > 0 ? kLanePhotonsHole : kLanePhotons;
+    plan.warps = (uint32_t)max((uint64_t)few, min((uint64_t)warps, num / (32 * per_lane)));
     const uint64_t lanes = 32ull * plan.warps;
     plan.groups = num >= kScreenFrom * lanes ? (int)min((uint64_t)kScreenGroups, num / lanes) : 0;
     plan.deal = num < lanes ? (int)((num + plan.warps - 1) / plan.warps) : -1;
@@ -1353,7 +1358,8 @@ __device__ __forceinline__ long long charge_bin(const ppcb_hit& h, uint32_t even
 // recorded hit is reached again.  A replay that does not end on the recorded hit (same
 // DOM, same time bits) is counted in stats[1].
 template <int MODEL>
-__global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_constant__ KArgs a, const ppcb_hit* __restrict__ hits,
+__global__ void __launch_bounds__(256, kAdjointPerSm) k_adjoint(const __grid_constant__ KArgs a,
+                                                 const ppcb_hit* __restrict__ hits,
                                                  const Prov* __restrict__ prov, uint64_t cap,
                                                  const unsigned long long* nh_dev, uint32_t events,
                                                  const float* __restrict__ wdom, const float2* __restrict__ wgrad,

@@ -54,7 +54,8 @@ void** __cudaRegisterFatBinary(void*) {
 }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
+void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*,
+                            int*) {
   names[host] = name;
 }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}

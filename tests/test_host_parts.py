@@ -103,7 +103,10 @@ int main() {
     for (float x : {INFINITY, -INFINITY, NAN, 1e30f, -1e30f, 3e38f, -3e38f, 0.f}) check(x);
     for (int k = 0; k < lnum; k++) {
       float a = lr[k], b = lr[k];
-      for (int i = 0; i < 8; i++, a = std::nextafterf(a, INFINITY), b = std::nextafterf(b, -INFINITY)) check(a), check(b);
+      for (int i = 0; i < 8; i++) {
+        check(a), check(b);
+        a = std::nextafterf(a, INFINITY), b = std::nextafterf(b, -INFINITY);
+      }
     }
     for (int c = -2; c < 2 * kTiltCells + 2; c++) {  // the cells' edges and centres
       const float x = (float)((f.off - c / (2.0 * (kTiltCells - 1))) / -f.scale);
