@@ -37,7 +37,6 @@ struct LlhDevice {
   unsigned int* work = nullptr;
   double* partial = nullptr;         // [shift][CTA] sums of llf terms
   int* errors = nullptr;
-  int ndt_cap = 0;
   CallBuffers io;                    // host-pointer evaluations
   ~LlhDevice() {
     for (void* p : {(void*)dom_slot, (void*)doms, (void*)bin_block, (void*)block_dat, (void*)block_dom, (void*)win,
@@ -355,13 +354,22 @@ void count_prepare() {
   done.fetch_or(bit);
 }
 
+// CTAs of k_llh_terms per shift.
+int term_ctas(int nblocks) { return std::max(1, (nblocks + kThreads - 1) / kThreads); }
+
+// The counters of an evaluation of ndt shifts in 4-byte words: no-hit total, tickets, blocks x
+// shifts, DOMs x shifts (ndom = 0 without norm).
+size_t work_words(int ndt, int nblocks, int ndom) {
+  return 2 + (size_t)(ndt + 1) / 2 * 2 + ((size_t)ndt * nblocks + 1) / 2 * 2 + (size_t)ndt * ndom;
+}
+
 }  // namespace
 
 void Likelihood::upload() {
   cuda_dev_ = eng_.devs.at(dev_).dev;
   check(cudaSetDevice(cuda_dev_), "cudaSetDevice");
-  d_.reset(new LlhDevice);
-  LlhDevice& D = *d_;
+  std::unique_ptr<LlhDevice, LlhDeviceFree> d(new LlhDevice);
+  LlhDevice& D = *d;
   std::vector<double> dat(blocks.size());
   for (size_t k = 0; k < blocks.size(); k++) dat[k] = blocks[k].dat;
   D.dom_slot = upload_vec(dom_slot, "likelihood tables");
@@ -374,7 +382,14 @@ void Likelihood::upload() {
   D.win = upload_vec(w, "likelihood tables");
   check(cudaMalloc((void**)&D.errors, sizeof(int)), "likelihood scratch");
   check(cudaMemset(D.errors, 0, sizeof(int)), "likelihood scratch");
+  // scratch for any number of shifts: what a graph holds stays as long as the object
+  const int nblocks = (int)blocks.size();
+  check(cudaMalloc((void**)&D.work, work_words(PPCB_LLH_MAX_SHIFTS, nblocks, opts.norm ? (int)doms.size() : 0) *
+                                        sizeof(unsigned int)), "likelihood scratch");
+  check(cudaMalloc((void**)&D.partial, (size_t)PPCB_LLH_MAX_SHIFTS * term_ctas(nblocks) * sizeof(double)),
+        "likelihood scratch");
   count_prepare();
+  d_ = std::move(d);
 }
 
 Likelihood::~Likelihood() {
@@ -393,28 +408,14 @@ void Likelihood::eval_device(const ppcb_hit* dhits, uint64_t n, uint32_t seed, c
   check(cudaSetDevice(eng_.devs.at(dev_).dev), "cudaSetDevice");
   LlhDevice& D = *d_;
   const int nblocks = (int)blocks.size(), ndom = (int)doms.size();
-  const int parts = std::max(1, (nblocks + kThreads - 1) / kThreads);
-  // the evaluation's counters: no-hit total, tickets, blocks x shifts, DOMs x shifts with norm
+  const int parts = term_ctas(nblocks);
   const size_t ntick = (ndt + 1) / 2 * 2, nsimc = ((size_t)ndt * nblocks + 1) / 2 * 2;
-  auto words = [&](int m) {
-    return 2 + (size_t)(m + 1) / 2 * 2 + ((size_t)m * nblocks + 1) / 2 * 2 + (opts.norm ? (size_t)m * ndom : 0);
-  };
-  if (ndt > D.ndt_cap) {
-    for (void** p : {(void**)&D.work, (void**)&D.partial})
-      if (*p) {
-        cudaFree(*p);
-        *p = nullptr;
-      }
-    D.ndt_cap = 0;
-    check(cudaMalloc((void**)&D.work, words(ndt) * sizeof(unsigned int)), "likelihood scratch");
-    check(cudaMalloc((void**)&D.partial, (size_t)ndt * parts * sizeof(double)), "likelihood scratch");
-    D.ndt_cap = ndt;
-  }
   unsigned long long* nohit = reinterpret_cast<unsigned long long*>(D.work);
   unsigned int* ticket = D.work + 2;
   unsigned int* simc = ticket + ntick;
   unsigned int* stot = simc + nsimc;
-  check(cudaMemsetAsync(D.work, 0, words(ndt) * sizeof(unsigned int), st), "memset");
+  check(cudaMemsetAsync(D.work, 0, work_words(ndt, nblocks, opts.norm ? ndom : 0) * sizeof(unsigned int), st),
+        "memset");
   // where the counters are: with all shifts or a part of them in shared memory, or in global memory
   const size_t per_shift = std::max(1, nblocks + (opts.norm ? ndom : 0));
   const size_t parts_needed = (per_shift * ndt * sizeof(unsigned int) + kCountSmem - 1) / kCountSmem;

@@ -103,9 +103,9 @@ def test_attributes_are_set_before_a_capture(fake, what, kind, opts, request):
 
 @pytest.mark.parametrize("doms", [60, 400])
 def test_likelihood_scratch_does_not_follow_the_hits(fake, ice_full2d, doms):
-    """An evaluation's device memory is what the shifts need, whatever the number of hits: a
-    later call of more hits gives nothing back that a captured call would still write to."""
-    first, then = _run(fake, ice_full2d, """
+    """An evaluation's device memory does not depend on the number of hits or shifts: a later call
+    of more gives nothing back that a captured call would still write to."""
+    sizes = _run(fake, ice_full2d, """
 c = ctx()
 dom, per = np.repeat(np.arange(%d), 20), np.tile(np.arange(20), %d)
 d = np.zeros(len(dom), T.LLH_HIT_DTYPE)
@@ -113,12 +113,13 @@ d["str"], d["om"], d["t"], d["q"] = dom // 60 + 1, dom %% 60 + 1, 100.0 + 50.0 *
 L = Likelihood(c, d, lbin=25.0)
 assert L.info()["blocks"] > 768  # 64 shifts' counters are more than one CTA's shared memory
 dts, h, out = np.linspace(-100, 100, 64), np.zeros(5000, T.HIT_DTYPE), np.zeros(64)
+L.eval_device(h.ctypes.data, 10, dts[:5], 1.0, out.ctypes.data)  # and the back end's tables
 result = []
-for n in (1000, 5000):
-    L.eval_device(h.ctypes.data, n, dts, 1.0, out.ctypes.data)
+for n, ndt in ((1000, 5), (1000, 64), (5000, 64)):
+    L.eval_device(h.ctypes.data, n, dts[:ndt], 1.0, out.ctypes.data)
     result.append(rt.fake_device())
 """ % (doms, doms))
-    assert first == then
+    assert sizes[0] == sizes[1] == sizes[2]
 
 
 @pytest.mark.parametrize("given", ["observed", "weights"])
