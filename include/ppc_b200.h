@@ -274,7 +274,9 @@ int ppcb_propagate_noalloc(ppcb_ctx* c, int device, const ppcb_bunch* bunches, i
  * instead of the host's shared sequence: the same decisions in distribution, not hit by
  * hit.  Accepted hits are written in input order.
  * ppcb_accept_device: device pointers on `stream`; *count (a device pointer) receives the
- * number accepted; `out` must hold n records.  ppcb_accept: host buffers, device 0; at most
+ * number accepted; `out` must hold n records.  The context's scratch grows with n: a call of
+ * more hits than any before gives the smaller one back, so a graph that holds this call (or
+ * ppcb_sources_device) is captured after a call of the largest n.  ppcb_accept: host buffers, device 0; at most
  * `cap` records written, *nout receives the number accepted. */
 int ppcb_accept_device(ppcb_ctx* c, int device, const ppcb_hit* hits, uint64_t n, uint32_t seed, ppcb_acc_hit* out,
                        unsigned long long* count, void* stream);
