@@ -91,6 +91,40 @@ __device__ __noinline__ double src_proposal(double xm, float x, double* t) {
   return um;
 }
 
+struct SrcCount {
+  unsigned long long num;
+  bool err;
+};
+
+// The reference's rejection loop (gpu/f2k.cxx:412-431), for means from 12.  The stream is not
+// drawn from again, so it goes by value: by reference it would live in memory, here and in the
+// screened loop.
+__device__ __noinline__ SrcCount src_poisson_exact(double xm, SrcRng r) {
+  const double sq = sqrt(2 * xm), alxm = log(xm), g = xm * alxm - src_gammln(xm + 1);
+  for (int it = 0; it < kMaxTries; it++) {
+    double y, em;
+    int k = 0;
+    do {
+      y = tan((double)(PPCB_FPI * r.u()));
+      em = sq * y + xm;
+    } while (em < 0 && ++k < kMaxTries);
+    if (em < 0) break;
+    const double um = floor(em);
+    const double t = 0.9 * (1 + y * y) * exp(um * alxm - src_gammln(um + 1) - g);
+    if (!(r.u() > t)) return SrcCount{(unsigned long long)um, false};
+  }
+  return SrcCount{(unsigned long long)floor(xm + 0.5), true};
+}
+
+// Means from which the screening below leaves so many proposals open that a warp with a few such
+// lanes is better off without it.  1e6 sources with and without it: means around 3.6e7 200 and 200
+// us, 7.2e7 220 and 197, 1.2e8 237 and 200, 3.6e8 312 and 198, log-uniform from 1e6 to 1e9 259 and 204.
+// At 4e7 mixtures that reach little beyond lose (1e1 to 1e8: 150 and 188).  Lanes of a warp
+// (log-uniform 1e4 to 1e9, 1e0 to 1e9): from 3 lanes 198 and 222, 4 209 and 232, 6 232 and 234, never
+// 230 and 204.
+constexpr double kExactMean = 1e8;
+constexpr int kExactLanes = 3;
+
 // Poisson sample of mean xm (gpu/f2k.cxx:402-433): multiplication of uniforms below 12,
 // rejection from a Lorentzian above.  A proposal is first evaluated in single precision, with
 // bounds on its error: y = tan(x) to 4 units in the last place (7e-7 with its product by
@@ -106,7 +140,8 @@ __device__ __noinline__ double src_proposal(double xm, float x, double* t) {
 // Bound by issue and by lanes that wait for the unluckiest of their warp: the counts of 1e6
 // sources take 80 us instead of 157 (a thread that goes on to its next source while others
 // still reject: 95 us, the loop's state costs more than the waiting).
-__device__ unsigned long long src_poisson(double xm, SrcRng& r, bool& err) {
+// `exact_warp`: without the screening.
+__device__ unsigned long long src_poisson(double xm, bool exact_warp, SrcRng& r, bool& err) {
   if (isnan(xm)) {
     err = true;
     return 0;
@@ -124,6 +159,11 @@ __device__ unsigned long long src_poisson(double xm, SrcRng& r, bool& err) {
       t *= r.u();
     }
     return um;
+  }
+  if (exact_warp) {
+    const SrcCount c = src_poisson_exact(xm, r);
+    err |= c.err;
+    return c.num;
   }
   const float mf = (float)xm, sq = sqrtf(2 * mf), rx = 1 / mf;
   int negative = 0;  // proposals below zero in a row
@@ -355,17 +395,22 @@ __global__ void __launch_bounds__(kThreads) k_src_count(SrcArgs A) {
              (unsigned int)min((uint64_t)kThreads, A.n - k0) * kSrcWords);
   __syncthreads();
   unsigned long long num = 0;
+  const ppcb_source& s = reinterpret_cast<const ppcb_source*>(in)[threadIdx.x];
+  SrcRng r{0, 0, 0};
+  double mean = 0;
+  bool err = false;
   if (k < A.n) {
-    const ppcb_source& s = reinterpret_cast<const ppcb_source*>(in)[threadIdx.x];
-    SrcRng r = src_stream(A.seed, k, A.rm, A.nmul);
+    r = src_stream(A.seed, k, A.rm, A.nmul);
     ppcb_bunch p;
-    bool err = false;
-    const double mean = src_bunch(s, A.eff, A.ovr, p, &r, err);
+    mean = src_bunch(s, A.eff, A.ovr, p, &r, err);
+  }
+  const bool exact_warp = __popc(__ballot_sync(0xffffffffu, mean >= kExactMean)) >= kExactLanes;
+  if (k < A.n) {
     if (mean < 0) {  // exact count
       if (!(s.amount >= 0) || s.amount >= 1.8e19) err = true;
       else num = (unsigned long long)s.amount;
     } else {
-      num = src_poisson(mean, r, err);
+      num = src_poisson(mean, exact_warp, r, err);
     }
     A.num[k] = num;
     if (err) atomicAdd(A.errors, 1);

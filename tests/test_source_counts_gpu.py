@@ -148,3 +148,21 @@ def test_failed_source_is_reported_once(ctx, n):
         ctx.sources(bad, seed=2)
     bunches, _, photons = ctx.sources(src, seed=2)
     assert len(bunches) == n and photons == 5 * n
+
+
+def test_counts_do_not_depend_on_the_neighbours(ctx):
+    """Warps with 0 to 31 sources above the mean from which a warp leaves the screening out, just
+    below and above it: the counts of the double-precision sampler (tolerance as above)."""
+    n = 32 * 600
+    info, src = ctx.info(), np.zeros(n, T.SOURCE_DTYPE)
+    k = np.arange(n)
+    large = k % 32 < np.array([0, 1, 2, 3, 4, 31])[k // 32 % 6]
+    mean = np.where(large, np.where(k % 2, 1.01e8, 6e8), np.array([0.5, 20.0, 1e3, 9.9e7])[k // 192 % 4])
+    src["kind"], src["n"], src["beta"], src["q"] = T.SRC_MOPO, [0, 0, 1], 1, k
+    src["amount"] = light = (mean * info["ovr"] / info["eff"]).astype(np.float32)
+    bunches, bstart, photons = ctx.sources(src, seed=8)
+    got = np.zeros(n, np.int64)
+    np.add.at(got, bunches["q"], bunches["num"].astype(np.int64))
+    m = (light * np.float32(info["eff"]) / np.float32(info["ovr"])).astype(np.float64)
+    ref = poisson(m, Streams(8, n, ctx.tables()["rm"]))
+    assert photons == got.sum() and int((got != ref)[m < 1e6].sum()) == 0 and int((got != ref).sum()) <= 20
